@@ -5,6 +5,7 @@
 #include <memory>
 
 #include "common.cuh"
+#include "small.cuh"
 #include "sweep.cuh"
 
 namespace nkg {
@@ -29,6 +30,15 @@ struct RefineWork {
     DeviceArray<double> x64, part, fix_part;
     DeviceArray<double> unit_part;                  // queued product: 2 per unit
     DeviceArray<unsigned char> sc;                  // BiScalars
+};
+
+// Buffers of the one-launch run of a small graph (small.cuh), kept between runs.
+struct SmallWork {
+    SmallPlan plan{};
+    unsigned ctas = 0;  // 0: not set up
+    DeviceArray<double> y0, y1, part;
+    DeviceArray<SmallState> st;
+    PinnedHost<SmallState> host;
 };
 
 // Sliced layout (SELL-32 with chunked long rows, see sweep.cuh) of one
@@ -145,6 +155,7 @@ struct nkg_graph {
 
     nkg::DeviceArray<double> trace;      // residual of sweep i at [i] (kTraceCapacity)
     int hot_tier_kb = -1;                // nkg_graph_options.hot_tier_kb
+    nkg::SmallWork small;
 
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr;
     std::atomic<int> cancel{0};
