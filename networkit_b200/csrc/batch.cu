@@ -483,10 +483,22 @@ __global__ void bt_fill(const GraphMeta *__restrict__ meta, const uint32_t *__re
 
 using namespace nkg;
 
+#include "batch_smem.cuh"
+
 struct BatchGraph {
     cudaGraphExec_t exec = nullptr;
     uint32_t cluster = 0, threads = 0, split = 0, variant = 0;
     uint64_t layout_gen = 0;
+};
+
+// How the batch is split between the two kernels in one precision: the graphs
+// for batch_smem_kernel and the others, each largest first.
+struct BatchSplit {
+    DeviceArray<uint32_t> big, smem;
+    uint32_t n_big = 0, n_smem = 0;
+    uint32_t cluster = 0, clusters = 0;  // smem launch shape
+    size_t smem_bytes = 0;
+    bool ready = false;
 };
 
 struct nkg_batch {
@@ -498,7 +510,6 @@ struct nkg_batch {
     std::vector<uint64_t> node_off;            // host copy (count+1)
     std::vector<GraphMeta> meta_h;
     DeviceArray<GraphMeta> meta;
-    DeviceArray<uint32_t> order;               // queue -> graph (arcs, descending)
     DeviceArray<uint32_t> perm, degc, rowlen, row_ptr, col;
     DeviceArray<uint32_t> slice_off, col_sell;
     uint32_t slices = 0, layout_split = 0;
@@ -507,10 +518,20 @@ struct nkg_batch {
     uint64_t slots = 0;
     DeviceArray<float> y32[2];
     DeviceArray<double> y64[2];
+    // Graphs that fit into shared memory (batch_smem.cuh).
+    std::vector<SmemMeta> smeta_h;
+    DeviceArray<SmemMeta> smeta;
+    DeviceArray<SmemItem> sitem;
+    DeviceArray<uint4> sarcs;
+    uint64_t s_entries = 0;                    // entries of their iterates
+    DeviceArray<float> sy32[2];
+    DeviceArray<double> sy64[2];
+    BatchSplit splits[2];                      // [FP32, FP64]
+    std::vector<uint32_t> order_h;             // graphs by arcs, descending
     DeviceArray<double> out_buf, residual;
     DeviceArray<unsigned long long> iterations;
     DeviceArray<unsigned long long> times;     // per graph: start, end (ns)
-    DeviceArray<unsigned int> counters;        // queue, floor stops
+    DeviceArray<unsigned int> counters;        // queue, floor stops, shared-memory queue
     DeviceArray<BatchParams> prm;
     PinnedHost<BatchParams> prm_h;
     nkg_batch_tuning tuning{};
@@ -564,6 +585,174 @@ void batch_layout(nkg_batch *b, uint32_t split) {
     NKG_CUDA(cudaStreamSynchronize(s));
     b->layout_split = split;
     ++b->layout_gen;
+}
+
+// Items and arcs of the graphs that fit into shared memory in FP32.
+void smem_layout(nkg_batch *b) {
+    if (b->smeta)
+        return;
+    cudaStream_t s = b->stream;
+    const uint32_t count = b->count;
+    b->smeta.alloc(count);
+    NKG_CUDA(cudaMemcpyAsync(b->smeta.get(), b->smeta_h.data(), count * sizeof(SmemMeta),
+                             cudaMemcpyHostToDevice, s));
+    smem_count<<<ceil_div(count, 128), 128, 0, s>>>(b->smeta.get(), count, smem_max_nodes<float>(),
+                                                    b->rowlen.get());
+    NKG_CUDA(cudaGetLastError());
+    NKG_CUDA(cudaMemcpyAsync(b->smeta_h.data(), b->smeta.get(), count * sizeof(SmemMeta),
+                             cudaMemcpyDeviceToHost, s));
+    NKG_CUDA(cudaStreamSynchronize(s));
+    uint64_t items = 0, entries = 0;
+    for (SmemMeta &m : b->smeta_h) {
+        m.item0 = static_cast<uint32_t>(items);
+        m.ybase = static_cast<uint32_t>(entries);
+        if (m.items)
+            entries += (static_cast<uint64_t>(m.n) + 3) / 4 * 4;
+        items += m.items;
+    }
+    require(items < 0xffffffffull && entries < 0xffffffffull, "too many rows");
+    b->s_entries = entries;
+    NKG_CUDA(cudaMemcpyAsync(b->smeta.get(), b->smeta_h.data(), count * sizeof(SmemMeta),
+                             cudaMemcpyHostToDevice, s));
+    if (items) {
+        DeviceArray<uint32_t> steps(items), off(items + 1), graph(items);
+        b->sitem.alloc(items);
+        smem_items<<<std::min<uint32_t>(count, 4096), 256, 0, s>>>(
+            b->smeta.get(), count, b->rowlen.get(), b->sitem.get(), steps.get(), graph.get());
+        NKG_CUDA(cudaGetLastError());
+        NKG_CUDA(cudaMemsetAsync(off.get(), 0, sizeof(uint32_t), s));
+        size_t tb = 0;
+        NKG_CUDA(cub::DeviceScan::InclusiveSum(nullptr, tb, steps.get(), off.get() + 1,
+                                               static_cast<int64_t>(items), s));
+        DeviceArray<unsigned char> tmp(tb);
+        NKG_CUDA(cub::DeviceScan::InclusiveSum(tmp.get(), tb, steps.get(), off.get() + 1,
+                                               static_cast<int64_t>(items), s));
+        const uint32_t total = read_scalar(off.get() + items, s);
+        b->sarcs.alloc(static_cast<size_t>(total) * 32);
+        smem_fill<<<num_sms(b->device) * 16, 256, 0, s>>>(
+            b->smeta.get(), graph.get(), static_cast<uint32_t>(items), off.get(), b->row_ptr.get(),
+            b->col.get(), b->sitem.get(), b->sarcs.get());
+        NKG_CUDA(cudaGetLastError());
+    }
+    NKG_CUDA(cudaStreamSynchronize(s));
+}
+
+cudaLaunchConfig_t smem_config(unsigned cluster, unsigned grid, size_t bytes, cudaStream_t s,
+                               cudaLaunchAttribute *attr) {
+    cudaLaunchConfig_t cfg = {};
+    attr->id = cudaLaunchAttributeClusterDimension;
+    attr->val.clusterDim.x = cluster;
+    attr->val.clusterDim.y = 1;
+    attr->val.clusterDim.z = 1;
+    cfg.blockDim = dim3(kSmemThreads);
+    cfg.gridDim = dim3(grid);
+    cfg.dynamicSmemBytes = bytes;
+    cfg.stream = s;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cfg;
+}
+
+// Which graphs run in shared memory in precision T, and with what clusters:
+// the size with the least estimated time of one sweep of every graph, the
+// larger of the largest graph's and the sum over the clusters' share. A sweep
+// of a graph on c CTAs is modelled as 1.2 us (2 us with a cluster barrier),
+// its arcs at 6 (8-byte values: 4) per clock and CTA at 1.9 GHz, and the copy
+// of its iterate at 60 GB/s x 1.9.
+template <typename T>
+void batch_split(nkg_batch *b) {
+    BatchSplit &S = b->splits[sizeof(T) == 8 ? 1 : 0];
+    if (S.ready)
+        return;
+    smem_layout(b);
+    std::vector<uint32_t> big, small;
+    uint32_t max_n = 0;
+    for (uint32_t i : b->order_h) {
+        const SmemMeta &m = b->smeta_h[i];
+        if (m.items && m.n <= smem_max_nodes<T>()) {
+            small.push_back(i);
+            max_n = std::max(max_n, m.n);
+        } else {
+            big.push_back(i);
+        }
+    }
+    S.n_big = static_cast<uint32_t>(big.size());
+    S.n_smem = static_cast<uint32_t>(small.size());
+    S.big.alloc(std::max<size_t>(big.size(), 1));
+    S.smem.alloc(std::max<size_t>(small.size(), 1));
+    cudaStream_t s = b->stream;
+    if (S.n_big)
+        NKG_CUDA(cudaMemcpyAsync(S.big.get(), big.data(), big.size() * 4, cudaMemcpyHostToDevice, s));
+    if (S.n_smem) {
+        NKG_CUDA(cudaMemcpyAsync(S.smem.get(), small.data(), small.size() * 4,
+                                 cudaMemcpyHostToDevice, s));
+        auto kfn = batch_smem_kernel<T>;
+        S.smem_bytes = (static_cast<size_t>(max_n) + 8) * sizeof(T) / 16 * 16 + 16;
+        NKG_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      static_cast<int>(S.smem_bytes)));
+        double best = 1e300;
+        for (unsigned c = 1; c <= kSmemMaxCluster; c *= 2) {
+            cudaLaunchAttribute attr;
+            const cudaLaunchConfig_t cfg = smem_config(c, c, S.smem_bytes, s, &attr);
+            int clusters = 0;
+            if (cudaOccupancyMaxActiveClusters(&clusters, kfn, &cfg) != cudaSuccess ||
+                clusters < 1) {
+                cudaGetLastError();
+                continue;
+            }
+            double sum = 0.0, most = 0.0;
+            for (uint32_t i : small) {
+                const SmemMeta &m = b->smeta_h[i];
+                const double us = (c > 1 ? 2.0 : 1.2) +
+                                  m.arcs / (c * 1900.0 * (sizeof(T) == 8 ? 4.0 : 6.0)) +
+                                  m.n * static_cast<double>(sizeof(T)) / 114000.0;
+                sum += us;
+                most = std::max(most, us);
+            }
+            const double est = std::max(most, sum / clusters);
+            if (est < best) {
+                best = est;
+                S.cluster = c;
+                S.clusters = std::min<uint32_t>(static_cast<uint32_t>(clusters), S.n_smem);
+            }
+        }
+        require(S.cluster > 0, "the shared-memory batch kernel does not fit on this GPU");
+    }
+    NKG_CUDA(cudaStreamSynchronize(s));
+    S.ready = true;
+}
+
+template <typename T>
+T *smem_buf(nkg_batch *b, int k);
+template <>
+float *smem_buf<float>(nkg_batch *b, int k) { return b->sy32[k].get(); }
+template <>
+double *smem_buf<double>(nkg_batch *b, int k) { return b->sy64[k].get(); }
+
+template <typename T>
+void smem_launch(nkg_batch *b, double *out) {
+    const BatchSplit &S = b->splits[sizeof(T) == 8 ? 1 : 0];
+    SmemArgs<T> a{};
+    a.meta = b->smeta.get();
+    a.order = S.smem.get();
+    a.item = b->sitem.get();
+    a.arcs = b->sarcs.get();
+    a.degc = b->degc.get();
+    a.perm = b->perm.get();
+    a.y0 = smem_buf<T>(b, 0);
+    a.y1 = smem_buf<T>(b, 1);
+    a.out = out;
+    a.iterations = b->iterations.get();
+    a.residual = b->residual.get();
+    a.times = b->times.get();
+    a.queue = b->counters.get() + 2;
+    a.floor_stops = b->counters.get() + 1;
+    a.prm = b->prm.get();
+    a.count = S.n_smem;
+    cudaLaunchAttribute attr;
+    const cudaLaunchConfig_t cfg =
+        smem_config(S.cluster, S.clusters * S.cluster, S.smem_bytes, b->stream, &attr);
+    NKG_CUDA(cudaLaunchKernelEx(&cfg, batch_smem_kernel<T>, a));
 }
 
 template <typename T, int TH, typename F>
@@ -624,10 +813,16 @@ bool batch_launch(nkg_batch *b, const nkg_batch_tuning &t, T *y0, T *y1, double 
         }
         if (check_only)
             return;
+        const BatchSplit &S = b->splits[sizeof(T) == 8 ? 1 : 0];
+        NKG_CUDA(cudaMemsetAsync(b->counters.get(), 0, 3 * sizeof(unsigned int), s));
+        if (S.n_smem)
+            smem_launch<T>(b, out);
+        if (!S.n_big)
+            return;
         cfg.gridDim = dim3(static_cast<unsigned>(clusters) * t.cluster);
         BatchArgs<T> a{};
         a.meta = b->meta.get();
-        a.order = b->order.get();
+        a.order = S.big.get();
         a.row_ptr = b->row_ptr.get();
         a.col = b->col.get();
         a.slice_off = b->slice_off.get();
@@ -643,9 +838,8 @@ bool batch_launch(nkg_batch *b, const nkg_batch_tuning &t, T *y0, T *y1, double 
         a.queue = b->counters.get();
         a.floor_stops = b->counters.get() + 1;
         a.prm = b->prm.get();
-        a.count = b->count;
+        a.count = S.n_big;
         a.total = b->total;
-        NKG_CUDA(cudaMemsetAsync(b->counters.get(), 0, 2 * sizeof(unsigned int), s));
         NKG_CUDA(cudaLaunchKernelEx(&cfg, kfn, a));
     });
     return ok;
@@ -673,6 +867,9 @@ void ensure_iterates<float>(nkg_batch *b) {
             y.alloc(static_cast<size_t>(b->total) + 1);
             NKG_CUDA(cudaMemsetAsync(y.get(), 0, (static_cast<size_t>(b->total) + 1) * 4, b->stream));
         }
+    for (auto &y : b->sy32)
+        if (!y)
+            y.alloc(std::max<uint64_t>(b->s_entries, 4));
 }
 template <>
 void ensure_iterates<double>(nkg_batch *b) {
@@ -681,6 +878,9 @@ void ensure_iterates<double>(nkg_batch *b) {
             y.alloc(static_cast<size_t>(b->total) + 1);
             NKG_CUDA(cudaMemsetAsync(y.get(), 0, (static_cast<size_t>(b->total) + 1) * 8, b->stream));
         }
+    for (auto &y : b->sy64)
+        if (!y)
+            y.alloc(std::max<uint64_t>(b->s_entries, 4));
 }
 
 template <typename T>
@@ -810,13 +1010,21 @@ nkg_batch *batch_create(uint32_t count, const uint64_t *node_off, const uint64_t
     std::iota(order.begin(), order.end(), 0u);
     std::stable_sort(order.begin(), order.end(),
                      [&](uint32_t x, uint32_t y) { return garcs[x] > garcs[y]; });
-    b->order.alloc(count);
-    NKG_CUDA(cudaMemcpyAsync(b->order.get(), order.data(), count * 4, cudaMemcpyHostToDevice, s));
+    b->smeta_h.resize(count);
+    for (uint32_t i = 0; i < count; ++i) {
+        SmemMeta &m = b->smeta_h[i];
+        std::memset(&m, 0, sizeof(m));
+        m.base = b->meta_h[i].base;
+        m.n = b->meta_h[i].n;
+        m.sinks = hs[i];
+        m.arcs = static_cast<uint32_t>(garcs[i]);
+    }
+    b->order_h = std::move(order);
     b->out_buf.alloc(total);
     b->residual.alloc(count);
     b->iterations.alloc(count);
     b->times.alloc(2 * static_cast<size_t>(count));
-    b->counters.alloc(2);
+    b->counters.alloc(3);
     b->prm.alloc(1);
     b->prm_h.alloc(1);
     b->tuning.cluster = 4;
@@ -877,7 +1085,10 @@ cudaGraphExec_t batch_graph(nkg_batch *b, const nkg_batch_tuning &t) {
 // One run of the captured batch graph with the given tuning; device ms.
 template <typename T>
 float batch_timed(nkg_batch *b, const nkg_batch_tuning &t) {
-    batch_layout(b, t.split);
+    batch_split<T>(b);
+    const BatchSplit &S = b->splits[sizeof(T) == 8 ? 1 : 0];
+    if (S.n_big)
+        batch_layout(b, t.split);
     ensure_iterates<T>(b);
     cudaGraphExec_t exec = batch_graph<T>(b, t);
     NKG_CUDA(cudaEventRecord(b->ev0, b->stream));
@@ -1023,7 +1234,6 @@ int nkg_batch_tune(nkg_batch *b, const nkg_pr_params *p, uint32_t sweeps,
                 best = t;
         }
         b->tuning = best;
-        batch_layout(b, best.split);
         if (n_results)
             *n_results = nres;
         if (best_out)
@@ -1089,7 +1299,8 @@ int nkg_batch_run(nkg_batch *b, const nkg_pr_params *p, double *scores_out, int 
             stats->residual = maxres;
             stats->ms_total = ms;
             stats->ms_iterations = ms;
-            stats->kernel_launches = 1;
+            const BatchSplit &S = b->splits[p->precision == NKG_PREC_FP64 ? 1 : 0];
+            stats->kernel_launches = (S.n_big ? 1 : 0) + (S.n_smem ? 1 : 0);
             if (p->precision == NKG_PREC_FP64)
                 stats->fp64_sweeps = sweeps;
             else
