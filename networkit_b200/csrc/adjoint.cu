@@ -369,7 +369,7 @@ __global__ void __launch_bounds__(THREADS, UNROLL > 8 ? 512 / THREADS : WEIGHTED
     }
 }
 
-// Split out-rows (one thread each, chunks in order), then the last CTA
+// Split out-rows (for_split_rows), then the last CTA
 // closes the sweep: residual, tel.lam_out for the next sweep, stopping test.
 template <bool WEIGHTED>
 __global__ void __launch_bounds__(kAdjThreads) adj_fix(AdjArgs a) {
@@ -385,10 +385,9 @@ __global__ void __launch_bounds__(kAdjThreads) adj_fix(AdjArgs a) {
         res += a.part[2 * static_cast<size_t>(i)];
         td += a.part[2 * static_cast<size_t>(i) + 1];
     }
-    uint32_t r;
-    double acc;
-    if (split_row_sum<kAdjThreads>(a.chunk_begin, a.chunk_val, a.n_long, a.n_vlong, r, acc))
-        adj_row<WEIGHTED>(a, r, acc, tdot, res, td);
+    for_split_rows<kAdjThreads, double>(
+        a.chunk_begin, a.chunk_val, a.n_long, a.n_vlong,
+        [&](uint32_t r, double acc) { adj_row<WEIGHTED>(a, r, acc, tdot, res, td); });
     res = block_sum<kAdjThreads>(res, s_red);
     td = block_sum<kAdjThreads>(td, s_red);
     if (threadIdx.x == 0) {

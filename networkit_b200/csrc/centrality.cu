@@ -59,6 +59,8 @@ struct CentArgs {
     const double *__restrict__ x_in;         // n+1 (x_in[n] = pad)
     double *__restrict__ x_out;              // n+1 (rows < n written)
     double *__restrict__ chunk_val;
+    const uint32_t *__restrict__ chunk_slot;
+    uint32_t n_hot;                          // rows with segment sums (hot.cuh)
     double *__restrict__ part;               // per work unit of the sweep
     double *__restrict__ fix_part;           // per fix-up CTA
     CentState *st;
@@ -147,9 +149,11 @@ __global__ void __launch_bounds__(THREADS, WEIGHTED || UNROLL > 8 ? 1024 / THREA
                         acc = __dadd_rn(acc, cent_term<MODE, WEIGHTED>(a, x[k], w[k]));
             }
             if (s < a.s_chunk) {
-                a.chunk_val[static_cast<size_t>(s) * 32 + lane] = acc;
+                a.chunk_val[chunk_slot_of(a.chunk_slot, s, lane)] = acc;
             } else {
                 const uint32_t r = a.n_long + (s - a.s_chunk) * 32 + lane;
+                if (!WEIGHTED)
+                    acc = with_segments(a.chunk_begin, a.chunk_val, a.n_hot, r, acc);
                 if (r < a.n)
                     cent_row<MODE>(a, r, acc, len_prev, sq);
             }
@@ -160,8 +164,7 @@ __global__ void __launch_bounds__(THREADS, WEIGHTED || UNROLL > 8 ? 1024 / THREA
     }
 }
 
-// Split rows (a warp for each row of many chunks, one thread for each other
-// row; split_row_sum), then the last CTA sums
+// Split rows (for_split_rows), then the last CTA sums
 // the squares in a fixed order and takes NumericTools::equal(length, old, tol).
 template <int MODE>
 __global__ void __launch_bounds__(kCentFix) cent_fix(CentArgs a) {
@@ -174,10 +177,9 @@ __global__ void __launch_bounds__(kCentFix) cent_fix(CentArgs a) {
     // The sweep's unit partials: a fixed share of the units per thread.
     for (uint32_t i = blockIdx.x * kCentFix + threadIdx.x; i < a.units; i += gridDim.x * kCentFix)
         sq += a.part[i];
-    uint32_t r;
-    double acc;
-    if (split_row_sum<kCentFix>(a.chunk_begin, a.chunk_val, a.n_long, a.n_vlong, r, acc))
-        cent_row<MODE>(a, r, acc, len_prev, sq);
+    for_split_rows<kCentFix, double>(
+        a.chunk_begin, a.chunk_val, a.n_long, a.n_vlong,
+        [&](uint32_t r, double acc) { cent_row<MODE>(a, r, acc, len_prev, sq); });
     sq = block_sum<kCentFix>(sq, s_red);
     if (threadIdx.x == 0) {
         a.fix_part[blockIdx.x] = sq;
@@ -282,7 +284,7 @@ CentResult cent_run(nkg_graph *g, const SellLayout &L, const double *w_sell, dou
     DeviceArray<uint32_t> unit_start(static_cast<size_t>(units) + 1);
     sell_units(L, units, unit_start.get(), s);
     DeviceArray<double> x[2] = {DeviceArray<double>(n + 1), DeviceArray<double>(n + 1)};
-    DeviceArray<double> chunk_val(static_cast<size_t>(L.s_chunk) * 32 + 1), part(units),
+    DeviceArray<double> chunk_val(L.chunk_sums() + 1), part(units),
         fix_part(fix_ctas);
     DeviceArray<CentState> st(1);
     CentResult R;
@@ -298,6 +300,10 @@ CentResult cent_run(nkg_graph *g, const SellLayout &L, const double *w_sell, dou
     a.unit_start = unit_start.get();
     a.chunk_begin = L.chunk_begin.get();
     a.chunk_val = chunk_val.get();
+    a.chunk_slot = L.chunk_slot.get();
+    a.n_hot = L.n_hot;
+    HotRun<double> hot;
+    hot.setup(L, sms, s);
     a.part = part.get();
     a.fix_part = fix_part.get();
     a.st = st.get();
@@ -317,6 +323,8 @@ CentResult cent_run(nkg_graph *g, const SellLayout &L, const double *w_sell, dou
         for (int k = 0; k < kSweepsPerGraph; ++k) {
             a.x_in = x[k & 1].get();
             a.x_out = x[(k + 1) & 1].get();
+            R.launches += hot.launch<MODE>(L, a.x_in, a.chunk_val, n, MODE == 0 ? 0.0 : -1.0, alpha,
+                                           &st.get()->done, s);
             kfn<<<ctas, kCentThreads, 0, s>>>(a);
             cent_fix<MODE><<<fix_ctas, kCentFix, 0, s>>>(a);
         }

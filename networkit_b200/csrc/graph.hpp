@@ -5,6 +5,7 @@
 #include <memory>
 
 #include "common.cuh"
+#include "hot.cuh"
 #include "small.cuh"
 #include "sweep.cuh"
 
@@ -45,6 +46,7 @@ struct SmallWork {
 // adjacency: the in-adjacency for the forward sweeps, the out-adjacency for
 // the adjoint.
 struct SellLayout {
+    uint32_t chunk = kChunk;            // arcs per chunk of a split row (chunk_for)
     uint32_t n_long = 0, n_vlong = 0, n_chunks = 0, s_chunk = 0, slices = 0;
     uint64_t slots = 0;
     DeviceArray<uint32_t> chunk_begin;  // n_long+1
@@ -52,15 +54,72 @@ struct SellLayout {
     DeviceArray<uint64_t> slice_cost;   // slices, inclusive prefix of slice costs
     DeviceArray<uint32_t> col_sell;     // slots
     DeviceArray<double> w_sell64;       // slots (weighted)
+    // Source blocks (hot.cuh; unweighted in-adjacency of large graphs): rows
+    // [0, n_hot) have segments, whose sums are chunk sums of the row (its
+    // first chunk sums, chunk_begin has n_hot + 1 entries); the chunks of the
+    // slices above are then of the other arcs, stored chunk i's sum going to
+    // chunk_slot[i] (s_chunk * 32 entries; empty: i).
+    uint32_t n_hot = 0, n_sums = 0;
+    DeviceArray<uint32_t> chunk_slot;
+    HotBlocks hot_blocks{};
+    uint32_t hot_slices = 0;
+    uint64_t hot_steps = 0;
+    DeviceArray<uint4> hot_arcs;        // 32 lanes x 8 arcs per step
+    DeviceArray<uint32_t> hot_off;      // hot_slices + 1
+    DeviceArray<uint32_t> hot_slot;     // 32 per slice
+    DeviceArray<uint64_t> hot_cost;     // hot_slices each for FP64 and FP32, inclusive prefixes
+    // Entries of a chunk-sum buffer.
+    size_t chunk_sums() const { return std::max<size_t>(static_cast<size_t>(s_chunk) * 32, n_sums); }
 };
+
+// The launches of hot_kernel over one layout in one precision; launch() does
+// nothing (and returns 0) where the layout has no blocks.
+template <typename T>
+struct HotRun {
+    unsigned ctas = 0;
+    DeviceArray<uint32_t> cta_start;
+    void setup(const SellLayout &L, unsigned sms, cudaStream_t s);
+    template <int MODE = 0>
+    unsigned launch(const SellLayout &L, const T *y, T *sums, uint32_t n, T pad, T alpha,
+                    const int *skip, cudaStream_t s) const {
+        if (!ctas)
+            return 0;
+        HotArgs<T> a{};
+        a.arcs = L.hot_arcs.get();
+        a.off = L.hot_off.get();
+        a.slot = L.hot_slot.get();
+        a.cta_start = cta_start.get();
+        a.y = y;
+        a.sums = sums;
+        a.skip = skip;
+        a.blocks = L.hot_blocks;
+        a.n = n;
+        a.pad = pad;
+        a.alpha = alpha;
+        NKG_CUDA(cudaFuncSetAttribute(hot_kernel<T, MODE>,
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      static_cast<int>(hot_bytes<T>())));
+        hot_kernel<T, MODE><<<ctas, kHotKernelThreads, hot_bytes<T>(), s>>>(a);
+        return 1;
+    }
+};
+
+// Rows of more than `chunk` arcs cut into chunks of that many in CSR order:
+// their number, those of more than kShortChunks chunks, the first chunk of
+// each (n_long + 1 entries). Returns the number of chunks.
+uint32_t row_chunks(const uint32_t *rowlen, uint32_t n, uint32_t chunk, uint32_t &n_long,
+                    uint32_t &n_vlong, DeviceArray<uint32_t> &chunk_begin, cudaStream_t s);
 
 // Build the sliced layout of a CSR whose n rows are sorted by length,
 // descending; the weight of entry k is w[w_index[k]] (w[k] without an index,
 // no weights when w is null). Padding slots hold pad_col (kNone: n, the zero
-// entry of an iterate of n + 1).
+// entry of an iterate of n + 1). `blocks`: unweighted, columns numbered as the
+// rows are; the layout may get source blocks. `scratch`: an array of `arcs`
+// entries that is no longer needed, or null.
 void build_sell(SellLayout &L, uint32_t n, const uint32_t *row_ptr, const uint32_t *col,
                 const double *w, const uint32_t *w_index, const uint32_t *rowlen, int device,
-                cudaStream_t s, uint32_t pad_col = kNone);
+                cudaStream_t s, uint32_t pad_col = kNone, bool blocks = false,
+                DeviceArray<uint32_t> *scratch = nullptr);
 // map[slot] = index[k] for the CSR entry k each slot of L holds (kNone for
 // padding slots).
 void build_slot_map(const SellLayout &L, uint32_t n, const uint32_t *row_ptr, const uint32_t *index,
@@ -102,6 +161,7 @@ struct Plane {
     DeviceArray<uint32_t> q_unit_start;
     DeviceArray<double> q_part;
     uint32_t q_units = 0;
+    HotRun<T> hot_run;           // source blocks (hot.cuh), before every sweep
     // The sweep's last CTA closes each iteration (no fix-up launch): graphs
     // with no split rows and at most kCloseInSweepUnits units.
     bool close_in_sweep = false;
@@ -133,6 +193,10 @@ struct nkg_graph {
 
     // Sliced layout of the sweep (the in-adjacency).
     nkg::SellLayout fw;
+    // Chunks of the long rows in CSR order for the sweeps that read the CSR
+    // (personalised PageRank), built on first use.
+    uint32_t rc_long = 0, rc_chunks = 0;
+    nkg::DeviceArray<uint32_t> rc_begin;
     int sweep_shape = 0;
     bool arc_sorted = false;
     bool w64src_stale = false;  // w64src predates nkg_graph_set_weights

@@ -203,9 +203,12 @@ __global__ void validate_and_count(const uint64_t *__restrict__ in_ptr,
 }
 
 // Sort key per original id: deleted nodes 0 (sorted last), existing nodes
-// in-degree + 1, or with `bucketed` degree_bucket(in-degree) + 1 (the stable
-// sort then keeps the caller's order inside a bucket). Counts sinks
-// (existing, out-degree 0).
+// in-degree + 1 with, below it, the bit length of the out-degree, so that the
+// nodes of one in-degree are ordered by how often they are gathered (sinks,
+// never gathered, last): gathers of the many low in-degree nodes then share
+// lines. With `bucketed` degree_bucket(in-degree) + 1 (the stable sort then
+// keeps the caller's order inside a bucket). Counts sinks (existing,
+// out-degree 0).
 __global__ void make_keys(const uint64_t *__restrict__ in_ptr, const uint32_t *__restrict__ outdeg,
                           const uint8_t *__restrict__ exists, uint64_t z, int bucketed,
                           uint32_t *__restrict__ keys, uint32_t *__restrict__ ids,
@@ -215,11 +218,13 @@ __global__ void make_keys(const uint64_t *__restrict__ in_ptr, const uint32_t *_
     if (i < z) {
         const bool ex = exists == nullptr || exists[i];
         const uint64_t d = in_ptr[i + 1] - in_ptr[i];
-        const uint32_t k = bucketed ? degree_bucket(static_cast<uint32_t>(d))
-                                    : static_cast<uint32_t>(d);
-        keys[i] = ex ? k + 1 : 0u;
+        const uint32_t o = outdeg[i];
+        uint32_t k = degree_bucket(static_cast<uint32_t>(d)) + 1;
+        if (!bucketed)  // 27 bits of in-degree (more is one class: all hubs), 5 of out-degree
+            k = (min(static_cast<uint32_t>(d), (1u << 27) - 2) + 1) << 5 | min(32u - __clz(o), 31u);
+        keys[i] = ex ? k : 0u;
         ids[i] = static_cast<uint32_t>(i);
-        sink = ex && outdeg[i] == 0;
+        sink = ex && o == 0;
     }
     const int c = __syncthreads_count(sink);
     if (threadIdx.x == 0 && c)
@@ -361,13 +366,13 @@ __global__ void relabel_rows(const uint32_t *__restrict__ perm, const uint64_t *
     }
 }
 
-// Rows longer than kChunk (a prefix, the rows are sorted by length) and, of
-// those, rows with more than kShortChunks chunks.
-__global__ void count_long(const uint32_t *__restrict__ rowlen, uint64_t n,
-                           unsigned long long *__restrict__ cnt) {
+// Rows longer than `split` arcs (a prefix: the rows are sorted by length, or by
+// length bucket with `split` a power of two), and rows longer than `vsplit`.
+__global__ void count_long(const uint32_t *__restrict__ rowlen, uint64_t n, uint32_t split,
+                           uint64_t vsplit, unsigned long long *__restrict__ cnt) {
     const uint64_t r = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x;
-    const bool lg = r < n && rowlen[r] > kChunk;
-    const bool vl = r < n && rowlen[r] > kChunk * kShortChunks;
+    const bool lg = r < n && rowlen[r] > split;
+    const bool vl = r < n && rowlen[r] > vsplit;
     const int a = __syncthreads_count(lg);
     const int b = __syncthreads_count(vl);
     if (threadIdx.x == 0) {
@@ -379,68 +384,439 @@ __global__ void count_long(const uint32_t *__restrict__ rowlen, uint64_t n,
 }
 
 __global__ void chunk_counts(const uint32_t *__restrict__ rowlen, uint32_t n_long,
-                             uint32_t *__restrict__ nch) {
+                             uint32_t chunk, uint32_t *__restrict__ nch) {
     const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r < n_long)
-        nch[r] = (rowlen[r] + kChunk - 1) / kChunk;
+        nch[r] = (rowlen[r] + chunk - 1) / chunk;
 }
 
-// chunk_row[k] = split row of chunk k, chunk_idx[k] = its index in that row.
+// First arc and length of every chunk of the rows [0, n_long), in row order.
 __global__ void expand_chunks(const uint32_t *__restrict__ chunk_begin, uint32_t n_long,
-                              uint32_t *__restrict__ chunk_row, uint32_t *__restrict__ chunk_idx) {
+                              uint32_t chunk, const uint32_t *__restrict__ row_ptr,
+                              uint32_t *__restrict__ vstart,
+                              uint32_t *__restrict__ vlen) {
     const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
     const int lane = threadIdx.x & 31;
     for (uint32_t r = warp; r < n_long; r += nwarps) {
         const uint32_t b = chunk_begin[r], e = chunk_begin[r + 1];
+        const uint32_t rs = row_ptr[r], re = row_ptr[r + 1];
         for (uint32_t k = b + lane; k < e; k += 32) {
-            chunk_row[k] = r;
-            chunk_idx[k] = k - b;
+            const uint32_t st = rs + (k - b) * chunk;
+            vstart[k] = st;
+            vlen[k] = min(chunk, re - st);
         }
     }
 }
 
-// Virtual row v of slice s / lane: its first arc and its length.
+// --- Source blocks (hot.cuh) ---
+
+// Sampled source blocks: counts[b] = how many of `samples` arcs, spread evenly
+// over [0, arcs), gather from block b (kMaxBlocks: past the last block).
+__global__ void block_sample(const uint32_t *__restrict__ col, uint64_t arcs, uint32_t samples,
+                             unsigned int *__restrict__ counts) {
+    __shared__ unsigned int h[kMaxBlocks + 1];
+    for (uint32_t i = threadIdx.x; i <= kMaxBlocks; i += blockDim.x)
+        h[i] = 0;
+    __syncthreads();
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < samples)
+        atomicAdd(h + min(col[arcs * i / samples] / kHotIds, kMaxBlocks), 1u);
+    __syncthreads();
+    for (uint32_t k = threadIdx.x; k <= kMaxBlocks; k += blockDim.x)
+        if (h[k])
+            atomicAdd(counts + k, h[k]);
+}
+
+// How many of `samples` arcs, spread evenly, lie in a segment of their row.
+__global__ void segment_sample(const uint32_t *__restrict__ row_ptr,
+                               const uint32_t *__restrict__ col, uint32_t n, uint64_t arcs,
+                               uint32_t samples, BlockPlan plan, unsigned int *__restrict__ count) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    bool in = false;
+    if (i < samples) {
+        const uint32_t a = static_cast<uint32_t>(arcs * i / samples);
+        uint32_t lo = 0, hi = n;  // last row with row_ptr[row] <= a
+        while (hi - lo > 1) {
+            const uint32_t mid = lo + (hi - lo) / 2;
+            if (row_ptr[mid] <= a)
+                lo = mid;
+            else
+                hi = mid;
+        }
+        in = col[a] / kHotIds < plan.blocks_of(row_ptr[lo + 1] - row_ptr[lo]);
+    }
+    const int c = __syncthreads_count(in);
+    if (threadIdx.x == 0 && c)
+        atomicAdd(count, static_cast<unsigned int>(c));
+}
+
+// Segments (blocks used, plus the rest) of every split row.
+__global__ void segment_counts(const uint32_t *__restrict__ rowlen, uint32_t n_long, BlockPlan plan,
+                               uint32_t *__restrict__ nseg) {
+    const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r < n_long)
+        nseg[r] = plan.blocks_of(rowlen[r]) + 1;
+}
+
+// Stable partition of the arcs of split rows by source block (block nb: the
+// rest), one warp (BIG 0) or one CTA (BIG 1) per row: every warp counts its
+// contiguous share of the row, the counts are scanned block by block, and a
+// second pass places the arcs. seg_cnt receives the row's segment lengths, the
+// last one (the arcs of no block) again in rest.
+constexpr int kPartThreads = 256;
+template <bool BIG>
+__global__ void __launch_bounds__(kPartThreads)
+    partition_rows(const uint32_t *__restrict__ row_ptr, const uint32_t *__restrict__ col,
+                   uint32_t r_begin, uint32_t r_end, BlockPlan plan,
+                   const uint32_t *__restrict__ seg_base, uint32_t *__restrict__ seg_cnt,
+                   uint32_t *__restrict__ rest, uint32_t *__restrict__ pcol) {
+    constexpr uint32_t kWarps = kPartThreads / 32;
+    constexpr uint32_t kAhead = BIG ? 8 : 4;  // 32-arc loads in flight
+    __shared__ uint32_t s_cnt[kWarps][32];
+    const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const uint32_t lt = (1u << lane) - 1u;
+    const uint32_t r0 = r_begin + (BIG ? blockIdx.x : blockIdx.x * kWarps + wid);
+    const uint32_t stride = BIG ? gridDim.x : gridDim.x * kWarps;
+    for (uint32_t r = r0; r < r_end; r += stride) {
+        const uint32_t rs = row_ptr[r], re = row_ptr[r + 1];
+        const uint32_t nb = plan.blocks_of(re - rs);
+        uint32_t b = rs, e = re;
+        if (BIG) {
+            const uint32_t per = ((re - rs + kWarps - 1) / kWarps + 31) & ~31u;
+            b = min(re, rs + wid * per);
+            e = min(re, b + per);
+        }
+        uint32_t *cnt = s_cnt[wid];
+        cnt[lane] = 0;
+        __syncwarp();
+        for (uint32_t k0 = b; k0 < e; k0 += 32 * kAhead) {
+            uint32_t blk[kAhead];
+#pragma unroll
+            for (uint32_t q = 0; q < kAhead; ++q) {
+                const uint32_t k = k0 + 32 * q + lane;
+                blk[q] = k < e ? min(col[k] / kHotIds, nb) : 32u;
+            }
+#pragma unroll
+            for (uint32_t q = 0; q < kAhead; ++q) {
+                const uint32_t m = __match_any_sync(0xffffffffu, blk[q]);
+                if (blk[q] < 32 && !(m & lt))
+                    cnt[blk[q]] += __popc(m);
+                __syncwarp();
+            }
+        }
+        // Exclusive offsets: block-major over the row, then warp order.
+        if (BIG) {
+            __syncthreads();
+            if (wid == 0) {
+                uint32_t tot = 0;
+                for (uint32_t w = 0; w < kWarps; ++w)
+                    tot += s_cnt[w][lane];
+                if (lane <= nb)
+                    seg_cnt[seg_base[r] + lane] = tot;
+                if (lane == nb)
+                    rest[r] = tot;
+                uint32_t inc = tot;
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t t = __shfl_up_sync(0xffffffffu, inc, o);
+                    if (lane >= static_cast<uint32_t>(o))
+                        inc += t;
+                }
+                uint32_t at = inc - tot;
+                for (uint32_t w = 0; w < kWarps; ++w) {
+                    const uint32_t c = s_cnt[w][lane];
+                    s_cnt[w][lane] = at;
+                    at += c;
+                }
+            }
+            __syncthreads();
+        } else {
+            const uint32_t tot = cnt[lane];
+            if (lane <= nb)
+                seg_cnt[seg_base[r] + lane] = tot;
+            if (lane == nb)
+                rest[r] = tot;
+            uint32_t inc = tot;
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t t = __shfl_up_sync(0xffffffffu, inc, o);
+                if (lane >= static_cast<uint32_t>(o))
+                    inc += t;
+            }
+            cnt[lane] = inc - tot;
+            __syncwarp();
+        }
+        for (uint32_t k0 = b; k0 < e; k0 += 32 * kAhead) {
+            uint32_t c[kAhead];
+#pragma unroll
+            for (uint32_t q = 0; q < kAhead; ++q)
+                c[q] = k0 + 32 * q + lane < e ? col[k0 + 32 * q + lane] : 0u;
+#pragma unroll
+            for (uint32_t q = 0; q < kAhead; ++q) {
+                const bool in = k0 + 32 * q + lane < e;
+                const uint32_t blk = in ? min(c[q] / kHotIds, nb) : 32u;
+                const uint32_t m = __match_any_sync(0xffffffffu, blk);
+                const uint32_t at = in ? cnt[blk] + __popc(m & lt) : 0u;
+                __syncwarp();
+                if (in) {
+                    pcol[rs + at] = c[q];
+                    if (!(m & lt))
+                        cnt[blk] += __popc(m);
+                }
+                __syncwarp();
+            }
+        }
+        if (BIG)
+            __syncthreads();
+        else
+            __syncwarp();
+    }
+}
+
+// Chunks of every segment: the arcs of no block are chunks in rows past kChunk
+// only (rows [0, n_long)); in the others they stay the row's lane.
+__global__ void segment_chunks(uint32_t n_hot, uint32_t n_long, uint32_t chunk,
+                               const uint32_t *__restrict__ seg_base,
+                               const uint32_t *__restrict__ seg_cnt, uint32_t *__restrict__ nch) {
+    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+    const uint32_t lane = threadIdx.x & 31;
+    for (uint32_t r = warp; r < n_hot; r += nwarps) {
+        const uint32_t sb = seg_base[r], ns = seg_base[r + 1] - sb;
+        if (lane < ns) {
+            const uint32_t per = lane == ns - 1 ? chunk : kHotChunk;
+            nch[sb + lane] =
+                lane == ns - 1 && r >= n_long ? 0u : (seg_cnt[sb + lane] + per - 1) / per;
+        }
+    }
+}
+
+// Chunks of the partitioned rows, in row order, then block order: first arc,
+// length (a segment's chunks are of equal length, give or take one arc) and
+// sort key (block, then longest first); the first chunk of every row; the
+// last row of more than kShortChunks chunks. One warp per row.
+__global__ void expand_segments(const uint32_t *__restrict__ row_ptr, uint32_t n_hot,
+                                uint32_t n_long, const uint32_t *__restrict__ seg_base,
+                                const uint32_t *__restrict__ seg_cnt,
+                                const uint32_t *__restrict__ seg_chunk,
+                                uint32_t *__restrict__ chunk_begin, uint32_t *__restrict__ vstart,
+                                uint32_t *__restrict__ vlen, uint32_t *__restrict__ key,
+                                uint32_t *__restrict__ id, unsigned int *__restrict__ vlong) {
+    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+    const uint32_t lane = threadIdx.x & 31;
+    for (uint32_t r = warp; r < n_hot; r += nwarps) {
+        const uint32_t sb = seg_base[r], ns = seg_base[r + 1] - sb;
+        const uint32_t cnt = lane < ns ? seg_cnt[sb + lane] : 0u;
+        uint32_t inc = cnt;
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t t = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= static_cast<uint32_t>(o))
+                inc += t;
+        }
+        const uint32_t start = row_ptr[r] + inc - cnt;
+        if (lane == 0) {
+            chunk_begin[r] = seg_chunk[sb];
+            if (r == n_hot - 1)
+                chunk_begin[n_hot] = seg_chunk[sb + ns];
+            if (r < n_long && seg_chunk[sb + ns] - seg_chunk[sb] > kShortChunks)
+                atomicMax(vlong, r + 1);
+        }
+        if (!cnt)
+            continue;
+        const uint32_t k0 = seg_chunk[sb + lane], nch = seg_chunk[sb + lane + 1] - k0;
+        const uint32_t blk = lane == ns - 1 ? kMaxBlocks : lane;
+        for (uint32_t i = 0; i < nch; ++i) {
+            const uint32_t a = static_cast<uint32_t>(static_cast<uint64_t>(cnt) * i / nch);
+            const uint32_t z = static_cast<uint32_t>(static_cast<uint64_t>(cnt) * (i + 1) / nch);
+            vstart[k0 + i] = start + a;
+            vlen[k0 + i] = z - a;
+            key[k0 + i] = (blk << 9) | (kChunk - (z - a));
+            id[k0 + i] = k0 + i;
+        }
+    }
+}
+
+// Rows longer than `split`, `chunk` and `big` (prefixes of the rows), and the
+// arcs of the first of these. One thread each.
+__global__ void row_bounds(const uint32_t *__restrict__ row_ptr, uint32_t n, uint32_t split,
+                           uint32_t chunk, uint32_t big, uint32_t *__restrict__ bounds) {
+    const uint32_t t = threadIdx.x;
+    if (t > 2)
+        return;
+    const uint32_t len = t == 0 ? split : t == 1 ? chunk : big;
+    uint32_t lo = 0, hi = n;
+    while (lo < hi) {
+        const uint32_t mid = lo + (hi - lo) / 2;
+        if (row_ptr[mid + 1] - row_ptr[mid] > len)
+            lo = mid + 1;
+        else
+            hi = mid;
+    }
+    bounds[t] = lo;
+    if (t == 0)
+        bounds[3] = row_ptr[lo];
+}
+
+// First chunk of every block in the sorted order (kMaxBlocks: the chunks of
+// no block; one past it: all), and *vlong after them. One thread per block.
+__global__ void block_bounds(const uint32_t *__restrict__ key, uint32_t n_chunks,
+                             const uint32_t *__restrict__ vlong, uint32_t *__restrict__ bounds) {
+    const uint32_t b = threadIdx.x;
+    if (b == kMaxBlocks + 2)
+        bounds[b] = *vlong;
+    if (b > kMaxBlocks + 1)
+        return;
+    uint32_t lo = 0, hi = n_chunks;
+    while (lo < hi) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (key[mid] < b << 9)
+            lo = mid + 1;
+        else
+            hi = mid;
+    }
+    bounds[b] = lo;
+}
+
+// Tables of the stored chunks first + [0, lanes) of which count exist: where
+// the sum goes (the others: an index past every sum's), first arc, length.
+__global__ void order_chunks(const uint32_t *__restrict__ order, uint32_t first, uint32_t count,
+                             uint32_t lanes, const uint32_t *__restrict__ vstart,
+                             const uint32_t *__restrict__ vlen, uint32_t spare,
+                             uint32_t *__restrict__ slot, uint32_t *__restrict__ vstart_s,
+                             uint32_t *__restrict__ vlen_s) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= lanes)
+        return;
+    if (i < count) {
+        const uint32_t k = order[first + i];
+        slot[i] = k;
+        vstart_s[i] = vstart[k];
+        vlen_s[i] = vlen[k];
+    } else {
+        slot[i] = spare;
+    }
+}
+
+// Chunks of every hot slice: block b's from chunk `chunk.first[b]` on, 32 per
+// slice.
+struct HotChunks {
+    uint32_t first[kMaxBlocks + 1];
+};
+__device__ __forceinline__ uint32_t hot_chunk(const HotBlocks &sl, const HotChunks &ch, uint32_t s,
+                                              uint32_t lane, uint32_t &block) {
+    uint32_t b = 0;
+    while (sl.first[b + 1] <= s)
+        ++b;
+    block = b;
+    const uint32_t k = ch.first[b] + (s - sl.first[b]) * 32 + lane;
+    return k < ch.first[b + 1] ? k : kNone;
+}
+
+// Steps of every hot slice (its first chunk is its longest) and its cost in
+// clocks in FP64 and FP32, fitted to the CTAs' times on R-MAT 22 and 24: 13 a
+// step, 24 a slice, 4.5 (FP32: 2) for every 32 arcs, 20,000 for a change of
+// block. One warp per slice.
+__global__ void hot_steps(HotBlocks sl, HotChunks ch, uint32_t slices,
+                          const uint32_t *__restrict__ order, const uint32_t *__restrict__ vlen,
+                          uint32_t *__restrict__ steps, uint64_t *__restrict__ cost64,
+                          uint64_t *__restrict__ cost32) {
+    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+    const uint32_t lane = threadIdx.x & 31;
+    for (uint32_t s = warp; s < slices; s += nwarps) {
+        uint32_t b;
+        const uint32_t k = hot_chunk(sl, ch, s, lane, b);
+        const uint32_t len = k != kNone ? vlen[order[k]] : 0u;
+        const uint32_t most = __shfl_sync(0xffffffffu, len, 0);
+        const uint32_t arcs = __reduce_add_sync(0xffffffffu, len);
+        if (lane == 0) {
+            const uint32_t n = (most + 7) / 8;
+            const uint32_t base = 13 * n + 24 + (s && s == sl.first[b] ? 20000u : 0u);
+            steps[s] = n;
+            cost64[s] = base + arcs * 9 / 64;
+            cost32[s] = base + arcs / 16;
+        }
+    }
+}
+
+// Arcs and sum slots of the hot slices (one warp each).
+__global__ void hot_fill(HotBlocks sl, HotChunks ch, uint32_t slices,
+                         const uint32_t *__restrict__ order, const uint32_t *__restrict__ vstart,
+                         const uint32_t *__restrict__ vlen, const uint32_t *__restrict__ pcol,
+                         const uint32_t *__restrict__ off, uint32_t *__restrict__ slot,
+                         uint4 *__restrict__ arcs) {
+    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+    const uint32_t lane = threadIdx.x & 31;
+    for (uint32_t s = warp; s < slices; s += nwarps) {
+        uint32_t b;
+        const uint32_t k = hot_chunk(sl, ch, s, lane, b);
+        const uint32_t id = k != kNone ? order[k] : kNone;
+        uint32_t p = 0, e = 0;
+        if (id != kNone) {
+            p = vstart[id];
+            e = p + vlen[id];
+        }
+        slot[s * 32 + lane] = id;
+        const uint32_t o = off[s], steps = off[s + 1] - o, base = b * kHotIds;
+#pragma unroll 2
+        for (uint32_t i = 0; i < steps; ++i, p += 8) {
+            uint32_t v[4];
+#pragma unroll
+            for (uint32_t j = 0; j < 4; ++j) {
+                const uint32_t lo = p + 2 * j < e ? pcol[p + 2 * j] - base : kHotIds;
+                const uint32_t hi = p + 2 * j + 1 < e ? pcol[p + 2 * j + 1] - base : kHotIds;
+                v[j] = lo | hi << 16;
+            }
+            arcs[(static_cast<size_t>(o) + i) * 32 + lane] = make_uint4(v[0], v[1], v[2], v[3]);
+        }
+    }
+}
+
+// Virtual row of slice s / lane: its first arc and its length. The chunks'
+// are tabulated in storage order. Rows [0, n_hot) keep their arcs of no block
+// only, the last rest[r] of the row in the partitioned order.
 struct VRow {
     uint32_t start;
     uint32_t len;
+    bool part;  // the arcs are those of the partitioned order
 };
 
-__device__ __forceinline__ VRow vrow_of(uint32_t s, int lane, uint32_t s_chunk, uint32_t n_chunks,
-                                        uint32_t n_long, uint32_t n,
-                                        const uint32_t *__restrict__ chunk_row,
-                                        const uint32_t *__restrict__ chunk_idx,
-                                        const uint32_t *__restrict__ row_ptr) {
-    VRow v{0, 0};
-    if (s < s_chunk) {
+struct VRows {
+    uint32_t s_chunk, n_chunks, n_long, n_hot, n;
+    const uint32_t *vstart, *vlen, *rest, *row_ptr;
+};
+
+__device__ __forceinline__ VRow vrow_of(uint32_t s, int lane, const VRows &t) {
+    VRow v{0, 0, t.n_hot != 0};
+    if (s < t.s_chunk) {
         const uint32_t k = s * 32 + lane;
-        if (k < n_chunks) {
-            const uint32_t r = chunk_row[k], c = chunk_idx[k];
-            const uint32_t rs = row_ptr[r], re = row_ptr[r + 1];
-            v.start = rs + c * kChunk;
-            v.len = min(kChunk, re - v.start);
+        if (k < t.n_chunks) {
+            v.start = t.vstart[k];
+            v.len = t.vlen[k];
         }
     } else {
-        const uint32_t r = n_long + (s - s_chunk) * 32 + lane;
-        if (r < n) {
-            v.start = row_ptr[r];
-            v.len = row_ptr[r + 1] - v.start;
+        const uint32_t r = t.n_long + (s - t.s_chunk) * 32 + lane;
+        if (r < t.n_hot) {
+            v.len = t.rest[r];
+            v.start = t.row_ptr[r + 1] - v.len;
+        } else if (r < t.n) {
+            v.start = t.row_ptr[r];
+            v.len = t.row_ptr[r + 1] - v.start;
+            v.part = false;
         }
     }
     return v;
 }
 
 // Slice length = longest of its 32 virtual rows (one warp per slice).
-__global__ void slice_lengths(uint32_t slices, uint32_t s_chunk, uint32_t n_chunks,
-                              uint32_t n_long, uint32_t n, const uint32_t *__restrict__ chunk_row,
-                              const uint32_t *__restrict__ chunk_idx,
-                              const uint32_t *__restrict__ row_ptr, uint32_t *__restrict__ slen,
+__global__ void slice_lengths(uint32_t slices, VRows t, uint32_t *__restrict__ slen,
                               uint64_t *__restrict__ scost) {
     const uint32_t s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (s >= slices)
         return;
-    const VRow v = vrow_of(s, lane, s_chunk, n_chunks, n_long, n, chunk_row, chunk_idx, row_ptr);
+    const VRow v = vrow_of(s, lane, t);
     uint32_t m = v.len;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1)
@@ -451,14 +827,12 @@ __global__ void slice_lengths(uint32_t slices, uint32_t s_chunk, uint32_t n_chun
     }
 }
 
-// Fill the column-major slices; padding slots point at the zero entry n. The
-// weight of CSR entry k is w[w_index[k]] (w[k] without an index); a null
-// col_sell refreshes the weights only.
-__global__ void fill_slices(uint32_t slices, uint32_t s_chunk, uint32_t n_chunks, uint32_t n_long,
-                            uint32_t n, const uint32_t *__restrict__ chunk_row,
-                            const uint32_t *__restrict__ chunk_idx,
-                            const uint32_t *__restrict__ row_ptr, const uint32_t *__restrict__ col,
-                            const double *__restrict__ w, const uint32_t *__restrict__ w_index,
+// Fill the column-major slices; padding slots point at the zero entry n. pcol:
+// the columns in the partitioned order (rows with source blocks). The weight
+// of CSR entry k is w[w_index[k]] (w[k] without an index).
+__global__ void fill_slices(uint32_t slices, VRows t, const uint32_t *__restrict__ col,
+                            const uint32_t *__restrict__ pcol, const double *__restrict__ w,
+                            const uint32_t *__restrict__ w_index,
                             const uint32_t *__restrict__ slice_off,
                             uint32_t *__restrict__ col_sell, double *__restrict__ w_sell,
                             uint32_t pad_col) {
@@ -466,14 +840,13 @@ __global__ void fill_slices(uint32_t slices, uint32_t s_chunk, uint32_t n_chunks
     const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
     const int lane = threadIdx.x & 31;
     for (uint32_t s = warp; s < slices; s += nwarps) {
-        const VRow v =
-            vrow_of(s, lane, s_chunk, n_chunks, n_long, n, chunk_row, chunk_idx, row_ptr);
+        const VRow v = vrow_of(s, lane, t);
         const uint32_t off = slice_off[s], len = slice_off[s + 1] - off;
+        const uint32_t *src = v.part ? pcol : col;
         for (uint32_t j = 0; j < len; ++j) {
             const size_t slot = (static_cast<size_t>(off) + j) * 32 + lane;
             const bool real = j < v.len;
-            if (col_sell)
-                col_sell[slot] = real ? col[v.start + j] : pad_col;
+            col_sell[slot] = real ? src[v.start + j] : pad_col;
             if (w_sell)
                 w_sell[slot] = real ? w[w_index ? w_index[v.start + j] : v.start + j] : 0.0;
         }
@@ -753,50 +1126,245 @@ static void sort_rows(nkg_graph *g, cudaStream_t s) {
     g->arc_sorted = true;
 }
 
-// Build the sliced layout L of a CSR whose n rows are sorted by length,
-// descending (row_ptr, col, optional weights w through w_index, rowlen).
-void build_sell(SellLayout &L, uint32_t n, const uint32_t *row_ptr, const uint32_t *col,
-                const double *w, const uint32_t *w_index, const uint32_t *rowlen, int device,
-                cudaStream_t s, uint32_t pad_col) {
-    if (pad_col == kNone)
-        pad_col = n;
-    const unsigned sms = num_sms(device);
+// Inclusive prefix sums of in[0, m) at out + 1, with out[0] = 0.
+static void scan_from_zero(const uint32_t *in, uint32_t *out, uint32_t m, cudaStream_t s) {
+    NKG_CUDA(cudaMemsetAsync(out, 0, sizeof(uint32_t), s));
+    size_t tb = 0;
+    NKG_CUDA(cub::DeviceScan::InclusiveSum(nullptr, tb, in, out + 1, static_cast<int64_t>(m), s));
+    DeviceArray<unsigned char> tmp(tb);
+    NKG_CUDA(cub::DeviceScan::InclusiveSum(tmp.get(), tb, in, out + 1, static_cast<int64_t>(m), s));
+}
+
+// Rows longer than `split` and rows of more than kShortChunks chunks of `split`.
+static void long_rows(const uint32_t *rowlen, uint32_t n, uint32_t split, uint32_t &n_long,
+                      uint32_t &n_vlong, cudaStream_t s) {
     DeviceArray<unsigned long long> cnt(2);
     NKG_CUDA(cudaMemsetAsync(cnt.get(), 0, 2 * sizeof(unsigned long long), s));
-    count_long<<<ceil_div(n, 256), 256, 0, s>>>(rowlen, n, cnt.get());
+    count_long<<<ceil_div(n, 256), 256, 0, s>>>(
+        rowlen, n, split, static_cast<uint64_t>(split) * kShortChunks, cnt.get());
     NKG_CUDA(cudaGetLastError());
     unsigned long long h_cnt[2];
     NKG_CUDA(cudaMemcpyAsync(h_cnt, cnt.get(), sizeof(h_cnt), cudaMemcpyDeviceToHost, s));
     NKG_CUDA(cudaStreamSynchronize(s));
-    L.n_long = static_cast<uint32_t>(h_cnt[0]);
-    L.n_vlong = static_cast<uint32_t>(h_cnt[1]);
+    n_long = static_cast<uint32_t>(h_cnt[0]);
+    n_vlong = static_cast<uint32_t>(h_cnt[1]);
+}
 
-    L.chunk_begin.alloc(static_cast<size_t>(L.n_long) + 1);
-    NKG_CUDA(cudaMemsetAsync(L.chunk_begin.get(), 0, sizeof(uint32_t), s));
-    DeviceArray<uint32_t> chunk_row, chunk_idx;
-    if (L.n_long) {
-        DeviceArray<uint32_t> nch(L.n_long);
-        chunk_counts<<<ceil_div(L.n_long, 256), 256, 0, s>>>(rowlen, L.n_long, nch.get());
-        size_t tb = 0;
-        NKG_CUDA(cub::DeviceScan::InclusiveSum(nullptr, tb, nch.get(), L.chunk_begin.get() + 1,
-                                               static_cast<int64_t>(L.n_long), s));
-        DeviceArray<unsigned char> tmp(tb);
-        NKG_CUDA(cub::DeviceScan::InclusiveSum(tmp.get(), tb, nch.get(), L.chunk_begin.get() + 1,
-                                               static_cast<int64_t>(L.n_long), s));
-        L.n_chunks = read_scalar(L.chunk_begin.get() + L.n_long, s);
-        chunk_row.alloc(L.n_chunks);
-        chunk_idx.alloc(L.n_chunks);
-        expand_chunks<<<sms * 4, 256, 0, s>>>(L.chunk_begin.get(), L.n_long, chunk_row.get(),
-                                              chunk_idx.get());
-        NKG_CUDA(cudaGetLastError());
-    } else {
-        L.n_chunks = 0;
+uint32_t row_chunks(const uint32_t *rowlen, uint32_t n, uint32_t chunk, uint32_t &n_long,
+                    uint32_t &n_vlong, DeviceArray<uint32_t> &chunk_begin, cudaStream_t s) {
+    long_rows(rowlen, n, chunk, n_long, n_vlong, s);
+    chunk_begin.alloc(static_cast<size_t>(n_long) + 1);
+    if (!n_long) {
+        NKG_CUDA(cudaMemsetAsync(chunk_begin.get(), 0, sizeof(uint32_t), s));
+        return 0;
     }
+    DeviceArray<uint32_t> nch(n_long);
+    chunk_counts<<<ceil_div(n_long, 256), 256, 0, s>>>(rowlen, n_long, chunk, nch.get());
+    NKG_CUDA(cudaGetLastError());
+    scan_from_zero(nch.get(), chunk_begin.get(), n_long, s);
+    return read_scalar(chunk_begin.get() + n_long, s);
+}
+
+// Which source blocks pay for this adjacency (BlockPlan, hot.cuh): the leading
+// blocks that enough sampled arcs gather from.
+static BlockPlan plan_blocks(uint32_t n, uint64_t arcs, const uint32_t *row_ptr,
+                             const uint32_t *col, cudaStream_t s) {
+    BlockPlan plan{};
+    constexpr uint32_t kSamples = 1u << 18;
+    if (n <= kHotIds || arcs < kHotGraphArcs)
+        return plan;
+    DeviceArray<unsigned int> counts(kMaxBlocks + 1);
+    NKG_CUDA(cudaMemsetAsync(counts.get(), 0, (kMaxBlocks + 1) * sizeof(unsigned int), s));
+    block_sample<<<kSamples / 1024, 1024, 0, s>>>(col, arcs, kSamples, counts.get());
+    NKG_CUDA(cudaGetLastError());
+    unsigned int h[kMaxBlocks + 1];
+    NKG_CUDA(cudaMemcpyAsync(h, counts.get(), sizeof(h), cudaMemcpyDeviceToHost, s));
+    NKG_CUDA(cudaStreamSynchronize(s));
+    uint32_t least = kHotRow + 1;
+    for (uint32_t b = 0; b < kMaxBlocks; ++b) {
+        const double share = static_cast<double>(h[b]) / kSamples;
+        if (share < 1.0 / kBlockShare ||
+            share * static_cast<double>(arcs) < static_cast<double>(kBlockMinArcs))
+            break;
+        least = std::max(least, static_cast<uint32_t>(std::ceil(kMinSegment / share)));
+        plan.min_len[b] = least;
+        plan.blocks = b + 1;
+    }
+    if (plan.blocks) {
+        // Worth it where at least 1/8 of the arcs become segments' (R-MAT 24:
+        // 0.5; Barabasi-Albert, whose few long rows hold few arcs: 0.02).
+        NKG_CUDA(cudaMemsetAsync(counts.get(), 0, sizeof(unsigned int), s));
+        segment_sample<<<kSamples / 256, 256, 0, s>>>(row_ptr, col, n, arcs, kSamples, plan,
+                                                      counts.get());
+        NKG_CUDA(cudaGetLastError());
+        if (read_scalar(counts.get(), s) < kSamples / 8)
+            plan.blocks = 0;
+    }
+    return plan;
+}
+
+// A table of the chunks of rows [0, n_long) in CSR order.
+static void plain_chunks(const SellLayout &L, const uint32_t *row_ptr, unsigned sms,
+                         DeviceArray<uint32_t> &vstart, DeviceArray<uint32_t> &vlen,
+                         cudaStream_t s) {
+    vstart.alloc(std::max<uint32_t>(L.n_chunks, 1));
+    vlen.alloc(std::max<uint32_t>(L.n_chunks, 1));
+    if (L.n_long) {
+        expand_chunks<<<sms * 4, 256, 0, s>>>(L.chunk_begin.get(), L.n_long, L.chunk, row_ptr,
+                                              vstart.get(), vlen.get());
+        NKG_CUDA(cudaGetLastError());
+    }
+}
+
+// Source blocks of L: partitions the arcs of rows [0, n_hot) (pcol, rest),
+// builds the hot slices, and tabulates the chunks of the other arcs of the
+// long rows (vstart, vlen, chunk_slot).
+static void build_blocks(SellLayout &L, const BlockPlan &plan, uint32_t n, const uint32_t *row_ptr,
+                         const uint32_t *col, const uint32_t *rowlen, unsigned sms,
+                         DeviceArray<uint32_t> &pcol, DeviceArray<uint32_t> &rest,
+                         DeviceArray<uint32_t> &vstart, DeviceArray<uint32_t> &vlen,
+                         cudaStream_t s) {
+    // Rows longer than a power of two are a prefix in either row order.
+    uint32_t split = kHotRow;
+    while (split < plan.min_len[0] - 1)
+        split *= 2;
+    split = std::min(split, L.chunk);  // the long rows are among the partitioned ones
+    DeviceArray<uint32_t> bounds(kMaxBlocks + 3);
+    row_bounds<<<1, 32, 0, s>>>(row_ptr, n, split, L.chunk, kBigRow, bounds.get());
+    NKG_CUDA(cudaGetLastError());
+    uint32_t hb[kMaxBlocks + 3];
+    NKG_CUDA(cudaMemcpyAsync(hb, bounds.get(), 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+    NKG_CUDA(cudaStreamSynchronize(s));
+    L.n_hot = hb[0];
+    L.n_long = hb[1];
+    const uint32_t big = hb[2], hot_rows_arcs = hb[3];
+    L.n_chunks = L.n_vlong = L.n_sums = 0;
+    L.chunk_begin.alloc(static_cast<size_t>(L.n_hot) + 1);
+    NKG_CUDA(cudaMemsetAsync(L.chunk_begin.get(), 0, sizeof(uint32_t), s));
+    if (!L.n_hot)
+        return;
+    // One block of scratch per size that becomes known (an allocation given
+    // back waits for the device).
+    const size_t rows = L.n_hot;
+    DeviceArray<uint32_t> by_row(2 * rows + 1);
+    uint32_t *nseg = by_row.get(), *seg_base = nseg + rows;
+    segment_counts<<<ceil_div(rows, 256), 256, 0, s>>>(rowlen, L.n_hot, plan, nseg);
+    NKG_CUDA(cudaGetLastError());
+    scan_from_zero(nseg, seg_base, L.n_hot, s);
+    const uint32_t segs = read_scalar(seg_base + rows, s);
+    DeviceArray<uint32_t> by_seg(3 * static_cast<size_t>(segs) + 1);
+    uint32_t *seg_cnt = by_seg.get(), *nch = seg_cnt + segs, *seg_chunk = nch + segs;
+    if (pcol.size() < hot_rows_arcs)
+        pcol.alloc(hot_rows_arcs);
+    rest.alloc(L.n_hot);
+    if (big)
+        partition_rows<true><<<std::min<unsigned>(big, sms * 8), kPartThreads, 0, s>>>(
+            row_ptr, col, 0, big, plan, seg_base, seg_cnt, rest.get(), pcol.get());
+    if (L.n_hot > big)
+        partition_rows<false>
+            <<<std::min<unsigned>(ceil_div(L.n_hot - big, kPartThreads / 32), sms * 16),
+               kPartThreads, 0, s>>>(row_ptr, col, big, L.n_hot, plan, seg_base, seg_cnt,
+                                     rest.get(), pcol.get());
+    segment_chunks<<<sms * 16, 256, 0, s>>>(L.n_hot, L.n_long, L.chunk, seg_base, seg_cnt, nch);
+    NKG_CUDA(cudaGetLastError());
+    scan_from_zero(nch, seg_chunk, segs, s);
+    const uint32_t chunks = read_scalar(seg_chunk + segs, s);
+    if (!chunks) {
+        L.n_hot = 0;
+        return;
+    }
+    DeviceArray<uint32_t> by_chunk(6 * static_cast<size_t>(chunks) + 1);
+    uint32_t *vs = by_chunk.get(), *vl = vs + chunks, *key = vl + chunks, *key_s = key + chunks,
+             *id = key_s + chunks, *order = id + chunks, *vlong = order + chunks;
+    NKG_CUDA(cudaMemsetAsync(vlong, 0, sizeof(uint32_t), s));
+    expand_segments<<<sms * 16, 256, 0, s>>>(row_ptr, L.n_hot, L.n_long, seg_base, seg_cnt,
+                                             seg_chunk, L.chunk_begin.get(), vs, vl, key, id, vlong);
+    NKG_CUDA(cudaGetLastError());
+    size_t tb = 0;
+    NKG_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb, key, key_s, id, order,
+                                             static_cast<int64_t>(chunks), 0, 14, s));
+    DeviceArray<unsigned char> tmp(tb);
+    NKG_CUDA(cub::DeviceRadixSort::SortPairs(tmp.get(), tb, key, key_s, id, order,
+                                             static_cast<int64_t>(chunks), 0, 14, s));
+    block_bounds<<<1, 64, 0, s>>>(key_s, chunks, vlong, bounds.get());
+    NKG_CUDA(cudaGetLastError());
+    NKG_CUDA(cudaMemcpyAsync(hb, bounds.get(), sizeof(hb), cudaMemcpyDeviceToHost, s));
+    NKG_CUDA(cudaStreamSynchronize(s));
+    L.n_vlong = hb[kMaxBlocks + 2];
+    HotChunks ch;
+    std::copy(hb, hb + kMaxBlocks + 1, ch.first);
+    L.hot_blocks.first[0] = 0;
+    for (uint32_t b = 0; b < kMaxBlocks; ++b)
+        L.hot_blocks.first[b + 1] = L.hot_blocks.first[b] + (hb[b + 1] - hb[b] + 31) / 32;
+    L.hot_slices = L.hot_blocks.first[kMaxBlocks];
+    // The chunks of no block, and one spare sum for the lanes past them.
+    L.n_chunks = chunks - hb[kMaxBlocks];
     L.s_chunk = (L.n_chunks + 31) / 32;
+    L.n_sums = chunks + 1;
+    const uint32_t lanes = L.s_chunk * 32;
+    L.chunk_slot.alloc(std::max<uint32_t>(lanes, 1));
+    vstart.alloc(std::max<uint32_t>(L.n_chunks, 1));
+    vlen.alloc(std::max<uint32_t>(L.n_chunks, 1));
+    if (lanes)
+        order_chunks<<<ceil_div(lanes, 256), 256, 0, s>>>(
+            order, hb[kMaxBlocks], L.n_chunks, lanes, vs, vl, chunks, L.chunk_slot.get(),
+            vstart.get(), vlen.get());
+    NKG_CUDA(cudaGetLastError());
+    if (!L.hot_slices)
+        return;
+    DeviceArray<uint32_t> steps(L.hot_slices);
+    DeviceArray<uint64_t> cost(2 * static_cast<size_t>(L.hot_slices));
+    L.hot_off.alloc(static_cast<size_t>(L.hot_slices) + 1);
+    L.hot_cost.alloc(2 * static_cast<size_t>(L.hot_slices));
+    L.hot_slot.alloc(static_cast<size_t>(L.hot_slices) * 32);
+    hot_steps<<<sms * 8, 256, 0, s>>>(L.hot_blocks, ch, L.hot_slices, order, vl, steps.get(),
+                                      cost.get(), cost.get() + L.hot_slices);
+    NKG_CUDA(cudaGetLastError());
+    scan_from_zero(steps.get(), L.hot_off.get(), L.hot_slices, s);
+    tb = 0;
+    NKG_CUDA(cub::DeviceScan::InclusiveSum(nullptr, tb, cost.get(), L.hot_cost.get(),
+                                           static_cast<int64_t>(L.hot_slices), s));
+    tmp.alloc(tb);
+    for (size_t at : {size_t{0}, static_cast<size_t>(L.hot_slices)})
+        NKG_CUDA(cub::DeviceScan::InclusiveSum(tmp.get(), tb, cost.get() + at, L.hot_cost.get() + at,
+                                               static_cast<int64_t>(L.hot_slices), s));
+    L.hot_steps = read_scalar(L.hot_off.get() + L.hot_slices, s);
+    L.hot_arcs.alloc(L.hot_steps * 32);
+    hot_fill<<<sms * 16, 256, 0, s>>>(L.hot_blocks, ch, L.hot_slices, order, vs, vl, pcol.get(),
+                                      L.hot_off.get(), L.hot_slot.get(), L.hot_arcs.get());
+    NKG_CUDA(cudaGetLastError());
+    NKG_CUDA(cudaStreamSynchronize(s));
+}
+
+// Build the sliced layout L of a CSR whose n rows are sorted by length,
+// descending (row_ptr, col, optional weights w through w_index, rowlen).
+void build_sell(SellLayout &L, uint32_t n, const uint32_t *row_ptr, const uint32_t *col,
+                const double *w, const uint32_t *w_index, const uint32_t *rowlen, int device,
+                cudaStream_t s, uint32_t pad_col, bool blocks, DeviceArray<uint32_t> *scratch) {
+    if (pad_col == kNone)
+        pad_col = n;
+    const unsigned sms = num_sms(device);
+    const uint32_t arcs = read_scalar(row_ptr + n, s);
+    L.chunk = chunk_for(arcs, sms);
+    BlockPlan plan{};
+    if (blocks && !w)
+        plan = plan_blocks(n, arcs, row_ptr, col, s);
+    DeviceArray<uint32_t> vstart, vlen, pcol, rest;
+    if (plan.blocks && scratch)
+        pcol = std::move(*scratch);
+    if (plan.blocks)
+        build_blocks(L, plan, n, row_ptr, col, rowlen, sms, pcol, rest, vstart, vlen, s);
+    if (!L.n_hot) {
+        L.n_chunks = row_chunks(rowlen, n, L.chunk, L.n_long, L.n_vlong, L.chunk_begin, s);
+        plain_chunks(L, row_ptr, sms, vstart, vlen, s);
+        L.s_chunk = (L.n_chunks + 31) / 32;
+    }
     const uint64_t s_rows = (static_cast<uint64_t>(n - L.n_long) + 31) / 32;
     const uint64_t slices = L.s_chunk + s_rows;
     require(slices < 0xffffffffull, "too many slices");
     L.slices = static_cast<uint32_t>(slices);
+    const VRows rows{L.s_chunk, L.n_chunks, L.n_long, L.n_hot, n, vstart.get(), vlen.get(),
+                     rest.get(), row_ptr};
 
     DeviceArray<uint32_t> slen(L.slices);
     DeviceArray<uint64_t> scost(L.slices);
@@ -804,8 +1372,7 @@ void build_sell(SellLayout &L, uint32_t n, const uint32_t *row_ptr, const uint32
     L.slice_off.alloc(static_cast<size_t>(L.slices) + 1);
     if (L.slices) {
         slice_lengths<<<ceil_div(static_cast<uint64_t>(L.slices) * 32, 256), 256, 0, s>>>(
-            L.slices, L.s_chunk, L.n_chunks, L.n_long, n, chunk_row.get(), chunk_idx.get(),
-            row_ptr, slen.get(), scost.get());
+            L.slices, rows, slen.get(), scost.get());
         NKG_CUDA(cudaGetLastError());
     }
     NKG_CUDA(cudaMemsetAsync(L.slice_off.get(), 0, sizeof(uint32_t), s));
@@ -828,9 +1395,8 @@ void build_sell(SellLayout &L, uint32_t n, const uint32_t *row_ptr, const uint32
     if (w)
         L.w_sell64.alloc(L.slots, 4);
     if (L.slices) {
-        fill_slices<<<sms * 16, 256, 0, s>>>(L.slices, L.s_chunk, L.n_chunks, L.n_long, n,
-                                             chunk_row.get(), chunk_idx.get(), row_ptr, col, w,
-                                             w_index, L.slice_off.get(), L.col_sell.get(),
+        fill_slices<<<sms * 16, 256, 0, s>>>(L.slices, rows, col, pcol.get(), w, w_index,
+                                             L.slice_off.get(), L.col_sell.get(),
                                              L.w_sell64.get(), pad_col);
         NKG_CUDA(cudaGetLastError());
     }
@@ -838,18 +1404,13 @@ void build_sell(SellLayout &L, uint32_t n, const uint32_t *row_ptr, const uint32
 }
 
 // map[slot] = index[k] for the CSR entry k the slot holds (kNone for padding).
-__global__ void fill_slot_map(uint32_t slices, uint32_t s_chunk, uint32_t n_chunks, uint32_t n_long,
-                              uint32_t n, const uint32_t *__restrict__ chunk_row,
-                              const uint32_t *__restrict__ chunk_idx,
-                              const uint32_t *__restrict__ row_ptr,
-                              const uint32_t *__restrict__ index,
+__global__ void fill_slot_map(uint32_t slices, VRows t, const uint32_t *__restrict__ index,
                               const uint32_t *__restrict__ slice_off, uint32_t *__restrict__ map) {
     const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
     const int lane = threadIdx.x & 31;
     for (uint32_t s = warp; s < slices; s += nwarps) {
-        const VRow v =
-            vrow_of(s, lane, s_chunk, n_chunks, n_long, n, chunk_row, chunk_idx, row_ptr);
+        const VRow v = vrow_of(s, lane, t);
         const uint32_t off = slice_off[s], len = slice_off[s + 1] - off;
         for (uint32_t j = 0; j < len; ++j)
             map[(static_cast<size_t>(off) + j) * 32 + lane] = j < v.len ? index[v.start + j] : kNone;
@@ -860,18 +1421,31 @@ void build_slot_map(const SellLayout &L, uint32_t n, const uint32_t *row_ptr, co
                     uint32_t *map, int device, cudaStream_t s) {
     if (!L.slices)
         return;
+    require(!L.n_hot, "internal: slot maps are of layouts without source blocks");
     const unsigned sms = num_sms(device);
-    DeviceArray<uint32_t> chunk_row(std::max<uint32_t>(L.n_chunks, 1)),
-        chunk_idx(std::max<uint32_t>(L.n_chunks, 1));
-    if (L.n_long)
-        expand_chunks<<<sms * 4, 256, 0, s>>>(L.chunk_begin.get(), L.n_long, chunk_row.get(),
-                                              chunk_idx.get());
-    fill_slot_map<<<sms * 16, 256, 0, s>>>(L.slices, L.s_chunk, L.n_chunks, L.n_long, n,
-                                           chunk_row.get(), chunk_idx.get(), row_ptr, index,
-                                           L.slice_off.get(), map);
+    DeviceArray<uint32_t> vstart, vlen;
+    plain_chunks(L, row_ptr, sms, vstart, vlen, s);
+    const VRows rows{L.s_chunk, L.n_chunks, L.n_long, 0, n, vstart.get(), vlen.get(), nullptr,
+                     row_ptr};
+    fill_slot_map<<<sms * 16, 256, 0, s>>>(L.slices, rows, index, L.slice_off.get(), map);
     NKG_CUDA(cudaGetLastError());
     NKG_CUDA(cudaStreamSynchronize(s));
 }
+
+template <typename T>
+void HotRun<T>::setup(const SellLayout &L, unsigned sms, cudaStream_t s) {
+    if (!L.hot_slices)
+        return;
+    const unsigned grid = sms;  // one CTA of a block's values per SM
+    cta_start.alloc(static_cast<size_t>(grid) + 1);
+    unit_bounds<<<ceil_div(static_cast<uint64_t>(grid) + 1, 256), 256, 0, s>>>(
+        L.hot_cost.get() + (sizeof(T) == 8 ? 0 : L.hot_slices), L.hot_slices, grid,
+        cta_start.get());
+    NKG_CUDA(cudaGetLastError());
+    ctas = grid;
+}
+template struct HotRun<double>;
+template struct HotRun<float>;
 
 // Cut the slices of L into `units` cost-balanced ranges (unit_start, units+1).
 void sell_units(const SellLayout &L, uint32_t units, uint32_t *unit_start, cudaStream_t s) {
@@ -1071,7 +1645,7 @@ static nkg_graph *build_graph(std::unique_ptr<nkg_graph> g, DeviceArray<uint64_t
             sort_rows(g.get(), s);
     }
     build_sell(g->fw, static_cast<uint32_t>(n), g->row_ptr.get(), g->col.get(), g->w64src.get(),
-               nullptr, rowlen.get(), dev, s);
+               nullptr, rowlen.get(), dev, s, kNone, true, &d_col);
     NKG_CUDA(cudaEventRecord(g->ev1, s));
     NKG_CUDA(cudaStreamSynchronize(s));
     float ms = 0.f;
@@ -1085,9 +1659,8 @@ static nkg_graph *build_graph(std::unique_ptr<nkg_graph> g, DeviceArray<uint64_t
     g->cta_sink.alloc(static_cast<size_t>(sms) * 32);
     // Fix-up grids also cover the queued sweep's unit partials (at most one
     // unit per slice, kUnitsPerFixThread per thread).
-    const size_t fix = std::max<size_t>(
-        static_cast<size_t>(g->fw.n_vlong) + ceil_div(g->fw.n_long, kFixThreads) + 1,
-        fix_ctas_with_units(1, g->fw.slices, kFixThreads));
+    const size_t fix = fix_ctas_with_units(split_fix_ctas<kFixThreads>(g->fw.n_long, g->fw.n_vlong),
+                                           g->fw.slices, kFixThreads);
     g->fix_res.alloc(fix);
     g->fix_sink.alloc(fix);
     g->rp.alloc(1);
@@ -1326,7 +1899,8 @@ static void sweep_setup(nkg_graph *g) {
         P.y[b].alloc(n + 1, 4);
         NKG_CUDA(cudaMemsetAsync(P.y[b].get(), 0, (n + 1 + 4) * sizeof(T), s));
     }
-    P.chunk_val.alloc(static_cast<size_t>(g->fw.s_chunk) * 32 + 1);
+    P.chunk_val.alloc(g->fw.chunk_sums() + 1);
+    P.hot_run.setup(g->fw, sms, s);
     if (WEIGHTED && !std::is_same<T, double>::value) {
         P.w_sell.alloc(g->fw.slots, 4);
         P.degw.alloc(n);
@@ -1355,8 +1929,7 @@ static void sweep_setup(nkg_graph *g) {
     unit_bounds<<<ceil_div(static_cast<uint64_t>(P.units) + 1, 256), 256, 0, s>>>(
         g->fw.slice_cost.get(), g->fw.slices, P.units, P.unit_start.get());
     NKG_CUDA(cudaGetLastError());
-    P.fix_ctas = fix_vlong_ctas(g->fw.n_vlong) +
-                 ceil_div(std::max<uint32_t>(g->fw.n_long - g->fw.n_vlong, 1), kFixThreads);
+    P.fix_ctas = split_fix_ctas<kFixThreads>(g->fw.n_long, g->fw.n_vlong);
     P.hot = hot_tier_ids<T>(g);
     if (!P.hot) {
         // The queued sweep's units (the tier kernel keeps the static ones).
@@ -1429,6 +2002,8 @@ static SweepArgs<T> sweep_args(nkg_graph *g, int in_buf) {
     a.y_in = P.y[in_buf].get();
     a.y_out = P.y[in_buf ^ 1].get();
     a.chunk_val = P.chunk_val.get();
+    a.chunk_slot = g->fw.chunk_slot.get();
+    a.n_hot = g->fw.n_hot;
     a.cta_res = g->cta_res.get();
     a.cta_sink = g->cta_sink.get();
     a.fix_res = g->fix_res.get();
@@ -1479,16 +2054,19 @@ template <typename T, bool WEIGHTED>
 static void launch_sweep(nkg_graph *g, int in_buf, cudaStream_t s) {
     Plane<T> &P = plane<T>(g);
     const SweepArgs<T> a = sweep_args<T, WEIGHTED>(g, in_buf);
+    P.hot_run.launch(g->fw, a.y_in, a.chunk_val, a.n, T(0), T(0), &a.st->done, s);
     launch_sweep_kernel<T, WEIGHTED>(g, a, s);
     if (!P.close_in_sweep)
         fixup_kernel<T, WEIGHTED><<<P.fix_ctas, kFixThreads, 0, s>>>(a);
 }
 
-// Kernel launches of one iteration: the sweep, and the fix-up unless the
-// sweep closes the iteration itself.
+// Kernel launches of one iteration: the segment sums where the layout has
+// source blocks, the sweep, and the fix-up unless the sweep closes the
+// iteration itself.
 template <typename T>
 static uint64_t launches_per_sweep(nkg_graph *g) {
-    return plane<T>(g).close_in_sweep ? 1 : 2;
+    const Plane<T> &P = plane<T>(g);
+    return (P.close_in_sweep ? 1 : 2) + (P.hot_run.ctas ? 1 : 0);
 }
 
 // Capture kSweepsPerGraph sweeps (sweep + fix-up each) as one CUDA graph.
@@ -1842,6 +2420,8 @@ static RunResult run_refine(nkg_graph *g, const nkg_pr_params &p, const double *
     a.degw = P32.degw.get();
     a.tele = P32.tele.get();
     a.chunk_val = P32.chunk_val.get();
+    a.chunk_slot = g->fw.chunk_slot.get();
+    a.n_hot = g->fw.n_hot;
     a.x = bx.get();
     a.r = br.get();
     a.rhat = brhat.get();
@@ -1884,10 +2464,13 @@ static RunResult run_refine(nkg_graph *g, const nkg_pr_params &p, const double *
     bl.d_sc = scp;
     bl.h_sc = hsc;
     bl.cancel = &g->cancel;
+    if (P32.hot_run.ctas)
+        bl.before_product = [&] {
+            return P32.hot_run.launch(g->fw, a.g, a.chunk_val, n, 0.f, 0.f, &scp->breakdown, s);
+        };
     // Solve (I - dM) x = r (r holds the right-hand side).
     auto solve = [&](double rel) { bi_solve<WEIGHTED, 0>(a, bl, rel, 0.25 * p.tol); };
 
-    cudaGraphExec_t exec = sweep_graph<double, WEIGHTED>(g, personal);
     IterState *sh = g->st_host.get();
     const double *degw64 = g->degw64src.get();
     bi_rhs_teleport<<<ceil_div(n, 256), 256, 0, s>>>(a);
@@ -1901,8 +2484,9 @@ static RunResult run_refine(nkg_graph *g, const nkg_pr_params &p, const double *
         bi_to_fp64<WEIGHTED><<<vec_ctas, kBiThreads, 0, s>>>(
             bx.get(), x64.get(), P64.y[0].get(), g->degc.get(), degw64, n, add, part.get(),
             g->st.get(), &scp->ticket, a.distribute, personal);
-        NKG_CUDA(cudaGraphLaunch(exec, s));
-        R.launches += 1 + launches_per_sweep<double>(g) * kSweepsPerGraph;
+        launch_sweep<double, WEIGHTED>(g, 0, s);
+        NKG_CUDA(cudaGetLastError());
+        R.launches += 1 + launches_per_sweep<double>(g);
         ++fp64;
         NKG_CUDA(cudaMemcpyAsync(sh, g->st.get(), sizeof(IterState), cudaMemcpyDeviceToHost, s));
         NKG_CUDA(cudaStreamSynchronize(s));
@@ -1998,6 +2582,7 @@ static void profile_sweeps(nkg_graph *g, int sweeps, double *ms_kernel, double *
     for (int i = 0; i < sweeps; ++i) {
         const SweepArgs<T> a = sweep_args<T, WEIGHTED>(g, i & 1);
         NKG_CUDA(cudaEventRecord(ev[2 * i], s));
+        P.hot_run.launch(g->fw, a.y_in, a.chunk_val, a.n, T(0), T(0), nullptr, s);
         launch_sweep_kernel<T, WEIGHTED>(g, a, s);
         NKG_CUDA(cudaEventRecord(ev[2 * i + 1], s));
         if (!P.close_in_sweep)
@@ -2060,15 +2645,21 @@ static double profile_gathers(nkg_graph *g, int reps) {
     const unsigned blocks = num_sms(g->device) * 8;
     DeviceArray<T> sink(static_cast<size_t>(blocks) * 256);
     const uint64_t slots = g->fw.slots;  // entries of col_sell
+    auto hot = [&](const T *y) {  // the gathers from shared memory
+        P.hot_run.launch(g->fw, y, P.chunk_val.get(), static_cast<uint32_t>(g->n), T(0), T(0),
+                         nullptr, s);
+    };
     cudaEvent_t e0, e1;
     NKG_CUDA(cudaEventCreate(&e0));
     NKG_CUDA(cudaEventCreate(&e1));
     gather_bound_kernel<T><<<blocks, 256, 0, s>>>(g->fw.col_sell.get(), slots, P.y[0].get(),
                                                   sink.get());  // warm-up
     NKG_CUDA(cudaEventRecord(e0, s));
-    for (int r = 0; r < reps; ++r)
+    for (int r = 0; r < reps; ++r) {
+        hot(P.y[r & 1].get());
         gather_bound_kernel<T><<<blocks, 256, 0, s>>>(g->fw.col_sell.get(), slots,
                                                       P.y[r & 1].get(), sink.get());
+    }
     NKG_CUDA(cudaEventRecord(e1, s));
     NKG_CUDA(cudaGetLastError());
     NKG_CUDA(cudaEventSynchronize(e1));
@@ -2226,7 +2817,7 @@ int nkg_graph_get_info(const nkg_graph *g, nkg_graph_info *info) {
         info->n = g->n;
         info->arcs = g->arcs;
         info->sinks = g->sinks;
-        info->slots = g->fw.slots;
+        info->slots = g->fw.slots + g->fw.hot_steps * 256;
         info->split_rows = g->fw.n_long;
         info->weighted = g->weighted;
         info->directed = g->directed;

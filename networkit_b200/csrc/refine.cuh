@@ -19,6 +19,8 @@
 // too), so rows are written in place.
 #pragma once
 
+#include <functional>
+
 #include <atomic>
 
 #include "sweep.cuh"
@@ -48,6 +50,8 @@ struct BiArgs {
     const float *__restrict__ degw;
     const float *__restrict__ tele;   // personalised teleport (n) or null
     float *__restrict__ chunk_val;
+    const uint32_t *__restrict__ chunk_slot;
+    uint32_t n_hot;                   // rows with segment sums (hot.cuh)
     // vectors (x-form, n entries; g is the gather form, n+1 with g[n] = 0;
     // for OP 1, p and s have n+1 entries with p[n] = s[n] = 0 and g is unused)
     float *x, *r, *rhat, *p, *v, *s, *t, *g;
@@ -169,9 +173,11 @@ __device__ __forceinline__ void bi_mv_unit(const BiArgs &a, const float *px, flo
                     acc += vv[k];
         }
         if (s < a.s_chunk) {
-            a.chunk_val[static_cast<size_t>(s) * 32 + lane] = acc;
+            a.chunk_val[chunk_slot_of(a.chunk_slot, s, lane)] = acc;
         } else {
             const uint32_t r = a.n_long + (s - a.s_chunk) * 32 + lane;
+            if (!WEIGHTED && OP == 0)
+                acc = with_segments(a.chunk_begin, a.chunk_val, a.n_hot, r, acc);
             if (r < a.n)
                 bi_mv_row<WEIGHTED, MODE, OP>(a, r, acc, px, out, d1, d2);
         }
@@ -240,10 +246,10 @@ __global__ void __launch_bounds__(kBiThreads) bi_mv_fix(BiArgs a) {
             d2 += a.unit_part[2 * static_cast<size_t>(i) + 1];
         }
     }
-    uint32_t r;
-    float acc;
-    if (split_row_sum<kBiThreads>(a.chunk_begin, a.chunk_val, a.n_long, a.n_vlong, r, acc))
-        bi_mv_row<WEIGHTED, MODE, OP>(a, r, acc, px, out, d1, d2);
+    for_split_rows<kBiThreads, float>(
+        a.chunk_begin, a.chunk_val, a.n_long, a.n_vlong, [&](uint32_t r, float acc) {
+            bi_mv_row<WEIGHTED, MODE, OP>(a, r, acc, px, out, d1, d2);
+        });
     d1 = block_sum<kBiThreads>(d1, s_red);
     d2 = block_sum<kBiThreads>(d2, s_red);
     if (threadIdx.x == 0) {
@@ -659,6 +665,9 @@ struct BiLaunch {
     BiScalars *d_sc = nullptr;    // device scalars
     BiScalars *h_sc = nullptr;    // pinned host copy
     std::atomic<int> *cancel = nullptr;
+    // Launches what a product needs before it (the segment sums of source
+    // blocks, hot.cuh); returns the kernels launched. Empty: nothing.
+    std::function<unsigned()> before_product;
     uint64_t launches = 0, matvecs = 0;
 };
 
@@ -684,6 +693,8 @@ void bi_solve(const BiArgs &a, BiLaunch &L, double rel, double floor) {
     for (int it = 0; it < 400 && !L.h_sc->breakdown && L.h_sc->res > inner_tol; it += 4) {
         for (int k = 0; k < 4; ++k) {
             bi_vec_p<WEIGHTED, OP><<<L.vec_ctas, kBiThreads, 0, s>>>(a);
+            if (L.before_product)
+                L.launches += L.before_product();
             with_sweep_shape(L.sweep_shape, [&](auto S) {
                 using Sh = decltype(S);
                 if (a.unit_part)
@@ -694,6 +705,8 @@ void bi_solve(const BiArgs &a, BiLaunch &L, double rel, double floor) {
             });
             bi_mv_fix<WEIGHTED, 0, OP><<<L.fix_ctas, kBiThreads, 0, s>>>(a);
             bi_vec_s<WEIGHTED, OP><<<L.vec_ctas, kBiThreads, 0, s>>>(a);
+            if (L.before_product)
+                L.launches += L.before_product();
             with_sweep_shape(L.sweep_shape, [&](auto S) {
                 using Sh = decltype(S);
                 if (a.unit_part)

@@ -13,7 +13,8 @@
 // Layout (SELL-C-sigma, Kreutzer et al., SIAM J. Sci. Comput. 36(5), 2014, with
 // C = 32 and sigma = n): nodes are relabelled by in-degree, descending, so 32
 // consecutive rows have nearly equal length. Rows longer than kChunk arcs are
-// cut into chunks of kChunk arcs ("virtual rows", placed first). Slice s holds
+// cut into chunks of kChunk arcs ("virtual rows", placed first); of rows with
+// source blocks (hot.cuh) only the arcs outside the blocks are here. Slice s holds
 // 32 virtual rows column-major: slot (j, lane) at col_sell[(off[s] + j) * 32 +
 // lane], so a warp loads 128 contiguous bytes per step and every lane sums its
 // own row sequentially, in the reference's arc order. No shared memory and no
@@ -26,19 +27,27 @@
 #pragma once
 
 #include <algorithm>
+#include <cmath>
 
 #include "common.cuh"
 
 namespace nkg {
 
-// Arcs per chunk of a split row; also the longest sequential loop of a lane.
-// Measured with the queued units (same box each): 512-arc chunks made R-MAT 24
-// (FP64) runs 0.9% faster (55,455 split rows instead of 190,051, a lighter
-// fix-up) but the weighted R-MAT 22 forward + backward 9% slower and the 4M
-// hyperbolic graph 1% slower; 128 was slower on R-MAT 24 too.
+// Arcs per chunk of a split row, which is also the longest sequential loop of a
+// lane (256 steps are 32 dependent batches). Graphs of less than 160 arcs for
+// every resident lane (7,104 warps) get shorter chunks, so that no warp ends
+// long after the others. Run times with chunks of 256 / 64 arcs, FP64: R-MAT
+// 23 34.1 / 36.7 ms, 22 21.0 / 21.7, 21 13.1 / 12.4; Barabasi-Albert of 64M
+// arcs 6.4 / 6.6.
 constexpr uint32_t kChunk = 256;
-// A split row with more chunks than this is summed by a whole warp in the fix-up.
-constexpr uint32_t kShortChunks = 16;
+constexpr uint32_t kSmallChunk = 64;
+inline uint32_t chunk_for(uint64_t arcs, unsigned sms) {
+    return arcs >= static_cast<uint64_t>(sms) * 48 * 32 * 160 ? kChunk : kSmallChunk;
+}
+// A split row with more chunk sums than this is summed by a whole warp in the
+// fix-up, the others by kRowLanes lanes.
+constexpr uint32_t kShortChunks = 128;
+constexpr uint32_t kRowLanes = 8;
 
 // Work units of the queued sweeps: warp gw of nw runs unit gw first, with no
 // ticket, then units nw + t for the tickets t it takes from `queue`, while
@@ -103,6 +112,10 @@ struct SweepArgs {
     const T *__restrict__ y_in;              // n+1 (y_in[n] = 0)
     T *__restrict__ y_out;
     T *__restrict__ chunk_val;               // per chunk slot: partial row sum
+    // Rows [0, n_hot) have segment sums of hot.cuh among their chunk sums
+    // (chunk_begin then has n_hot + 1 entries).
+    const uint32_t *__restrict__ chunk_slot; // where stored chunk i's sum goes (null: i)
+    uint32_t n_hot;
     double *__restrict__ cta_res;            // per sweep CTA
     double *__restrict__ cta_sink;
     double *__restrict__ fix_res;            // per fix-up CTA
@@ -141,6 +154,25 @@ struct SweepArgs {
 // Graphs with no split rows and at most this many units close every
 // iteration in the sweep's last CTA instead of a fix-up launch.
 constexpr uint32_t kCloseInSweepUnits = 8192;
+
+// Where the sum of chunk slice s / lane goes (chunk_slot null: storage order).
+__device__ __forceinline__ uint32_t chunk_slot_of(const uint32_t *chunk_slot, uint32_t s, int lane) {
+    const uint32_t i = s * 32 + lane;
+    return chunk_slot ? ld_stream(chunk_slot + i) : i;
+}
+
+// Adds the segment sums of row r (hot.cuh; written by the kernel before) to
+// the sum of its other arcs.
+template <typename V>
+__device__ __forceinline__ V with_segments(const uint32_t *__restrict__ chunk_begin,
+                                           const V *chunk_val, uint32_t n_hot, uint32_t r, V acc) {
+    if (r < n_hot) {
+        const uint32_t e = chunk_begin[r + 1];
+        for (uint32_t k = chunk_begin[r]; k < e; ++k)
+            acc += chunk_val[k];
+    }
+    return acc;
+}
 
 template <typename T>
 __device__ __forceinline__ T t_mul(T a, T b);
@@ -351,9 +383,11 @@ __device__ __forceinline__ void sweep_unit(const SweepArgs<T> &a, const T *s_y, 
                     acc += v[k];
         }
         if (s < a.s_chunk) {
-            a.chunk_val[static_cast<size_t>(s) * 32 + lane] = acc;
+            a.chunk_val[chunk_slot_of(a.chunk_slot, s, lane)] = acc;
         } else {
             const uint32_t r = a.n_long + (s - a.s_chunk) * 32 + lane;
+            if (!WEIGHTED && !PART)
+                acc = with_segments(a.chunk_begin, a.chunk_val, a.n_hot, r, acc);
             if (r < a.n)
                 finish_row_sweep<T, WEIGHTED, PART>(a, r, acc, res, sink);
         }
@@ -452,26 +486,20 @@ __global__ void __launch_bounds__(THREADS, UNROLL != 8 || (WEIGHTED && sizeof(T)
     }
 }
 
-// Fix-up: finish the split rows from their chunk sums (in chunk order), then
-// (last CTA) reduce all partial sums in index order and close the iteration
-// (PageRank.cpp:68-70). The first fix_vlong_ctas() CTAs finish the rows with
-// many chunks, one row per warp; the others take one split row per thread.
+// Fix-up: finish the split rows from their chunk sums, then (last CTA) reduce
+// all partial sums in index order and close the iteration
+// (PageRank.cpp:68-70).
 constexpr int kFixThreads = 256;
-constexpr uint32_t kFixWarps = kFixThreads / 32;
 
-__host__ __device__ inline uint32_t fix_vlong_ctas(uint32_t n_vlong) {
-    return (n_vlong + kFixWarps - 1) / kFixWarps;
-}
-
-// The same layout for the other fix-ups of split rows (FP32 product, adjoint,
-// centrality), with THREADS threads per CTA: the first CTAs give each row of
-// more than kShortChunks chunks a warp, the rest one thread per split row.
+// CTAs of THREADS threads that finish the split rows (for_split_rows): a warp
+// for each row of more than kShortChunks chunk sums, then kRowLanes lanes for
+// each other row, at most 8 CTAs per SM of them.
 template <int THREADS>
 inline unsigned split_fix_ctas(uint32_t n_long, uint32_t n_vlong) {
-    constexpr uint32_t w = THREADS / 32;
+    constexpr uint32_t w = THREADS / 32, rows = THREADS / kRowLanes;
     const uint64_t short_rows = n_long > n_vlong ? n_long - n_vlong : 0;
     return static_cast<unsigned>(std::max<uint64_t>(
-        1, (n_vlong + w - 1) / w + (short_rows + THREADS - 1) / THREADS));
+        1, (n_vlong + w - 1) / w + std::min<uint64_t>(1184, (short_rows + rows - 1) / rows)));
 }
 
 // Lane-strided partial sum of one split row's chunk partials
@@ -497,34 +525,53 @@ __device__ __forceinline__ V lane_chunk_sum(const V *__restrict__ v, uint32_t cb
     return part;
 }
 
-// Split row r of this thread in that layout and its chunk sum. Returns true
-// for the thread that finishes r (lane 0 of a row's warp, or the row's own
-// thread). A warp sums lane-strided partials in V, then across lanes in double
-// in a fixed tree; a thread sums the chunks in order. Every thread of a warp
-// given a row must call it (the lane sum is warp-wide).
-template <int THREADS, typename V>
-__device__ __forceinline__ bool split_row_sum(const uint32_t *__restrict__ chunk_begin,
-                                              const V *__restrict__ chunk_val, uint32_t n_long,
-                                              uint32_t n_vlong, uint32_t &r, V &acc) {
-    constexpr uint32_t w = THREADS / 32;
+// Calls finish(r, sum) once for every split row r < n_long with the sum of its
+// chunk sums, in a fixed order: a warp for each of the first n_vlong rows
+// (lane-strided partials in V, then across lanes in double), kRowLanes lanes
+// for each other (four loads of a lane in flight; one thread per row took 42
+// us of every R-MAT 24 iteration where source blocks give a row a dozen sums).
+// Every thread of the CTA calls it.
+template <int THREADS, typename V, typename F>
+__device__ __forceinline__ void for_split_rows(const uint32_t *__restrict__ chunk_begin,
+                                               const V *__restrict__ chunk_val, uint32_t n_long,
+                                               uint32_t n_vlong, F &&finish) {
+    constexpr uint32_t w = THREADS / 32, rows = THREADS / kRowLanes;
+    const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const uint32_t vctas = (n_vlong + w - 1) / w;
     if (blockIdx.x < vctas) {
-        r = blockIdx.x * w + (threadIdx.x >> 5);
+        const uint32_t r = blockIdx.x * w + wid;
         if (r >= n_vlong)
-            return false;
-        const int lane = threadIdx.x & 31;
-        const V part = lane_chunk_sum(chunk_val, chunk_begin[r], chunk_begin[r + 1], lane);
-        acc = static_cast<V>(warp_sum(static_cast<double>(part)));
-        return lane == 0;
+            return;
+        const V part = lane_chunk_sum(chunk_val, chunk_begin[r], chunk_begin[r + 1],
+                                      static_cast<int>(lane));
+        const V acc = static_cast<V>(warp_sum(static_cast<double>(part)));
+        if (lane == 0)
+            finish(r, acc);
+        return;
     }
-    r = n_vlong + (blockIdx.x - vctas) * THREADS + threadIdx.x;
-    if (r >= n_long)
-        return false;
-    V sum = V(0);
-    for (uint32_t k = chunk_begin[r]; k < chunk_begin[r + 1]; ++k)
-        sum += chunk_val[k];
-    acc = sum;
-    return true;
+    const uint32_t sub = lane % kRowLanes;
+    const uint32_t stride = (gridDim.x - vctas) * rows;
+    for (uint32_t base = n_vlong + (blockIdx.x - vctas) * rows + wid * (32 / kRowLanes);
+         base < n_long; base += stride) {
+        const uint32_t r = base + lane / kRowLanes;
+        const uint32_t e = r < n_long ? chunk_begin[r + 1] : 0u;
+        V sum = V(0);
+        for (uint32_t k = r < n_long ? chunk_begin[r] + sub : 0u; k < e; k += 4 * kRowLanes) {
+            V x[4];
+#pragma unroll
+            for (uint32_t q = 0; q < 4; ++q)
+                x[q] = k + q * kRowLanes < e ? chunk_val[k + q * kRowLanes] : V(0);
+#pragma unroll
+            for (uint32_t q = 0; q < 4; ++q)
+                sum += x[q];
+        }
+        __syncwarp();
+#pragma unroll
+        for (uint32_t o = kRowLanes / 2; o > 0; o >>= 1)
+            sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        if (sub == 0 && r < n_long)
+            finish(r, sum);
+    }
 }
 
 template <typename T, bool WEIGHTED, bool PART = false>
@@ -544,31 +591,10 @@ __global__ void __launch_bounds__(kFixThreads) fixup_kernel(SweepArgs<T> a) {
             sink += a.unit_sink[i];
         }
     }
-    const uint32_t vctas = fix_vlong_ctas(a.n_vlong);
-    if (blockIdx.x < vctas) {
-        const uint32_t r = blockIdx.x * kFixWarps + (threadIdx.x >> 5);
-        const int lane = threadIdx.x & 31;
-        if (r < a.n_vlong) {
-            const T part = lane_chunk_sum<T>(a.chunk_val, a.chunk_begin[r], a.chunk_begin[r + 1], lane);
-            const double tot = warp_sum(static_cast<double>(part));
-            if (lane == 0)
-                finish_row<T, WEIGHTED, PART>(a, rp, sink_coef, r, static_cast<T>(tot), res, sink);
-        }
-    } else {
-        const uint32_t r = a.n_vlong + (blockIdx.x - vctas) * kFixThreads + threadIdx.x;
-        if (r < a.n_long) {
-            const uint32_t cb = a.chunk_begin[r], ce = a.chunk_begin[r + 1];
-            T parts[kShortChunks];
-#pragma unroll
-            for (uint32_t k = 0; k < kShortChunks; ++k)
-                parts[k] = cb + k < ce ? a.chunk_val[cb + k] : T(0);
-            T sum = T(0);
-#pragma unroll
-            for (uint32_t k = 0; k < kShortChunks; ++k)
-                sum += parts[k];
+    for_split_rows<kFixThreads, T>(
+        a.chunk_begin, a.chunk_val, a.n_long, a.n_vlong, [&](uint32_t r, T sum) {
             finish_row<T, WEIGHTED, PART>(a, rp, sink_coef, r, sum, res, sink);
-        }
-    }
+        });
     const double bres = block_sum<kFixThreads>(res, s_red);
     const double bsink = block_sum<kFixThreads>(sink, s_red);
     if (threadIdx.x == 0) {

@@ -1,0 +1,97 @@
+"""Layouts whose long rows are grouped by source blocks (graphs of a few million
+arcs whose leading sources are gathered most) against the oracle: the plain and
+the centrality sweeps, the FP32 solve, weights and their gradients, and
+personalised PageRank, which reads the CSR itself."""
+import os
+
+import numpy as np
+import pytest
+
+from networkit_b200 import _capi, generators
+
+pytestmark = pytest.mark.gpu
+
+THREADS = os.cpu_count() or 1
+
+
+@pytest.fixture(scope="module")
+def rmat():
+    """R-MAT 22: large enough for source blocks, hubs of tens of thousands of
+    arcs (partitioned by a whole CTA)."""
+    csr = generators.rmat_directed(22, 12, seed=7)
+    dg = _capi.DeviceGraph(csr)
+    assert csr.arcs >= 40 << 20  # smaller graphs have none
+    return csr, dg
+
+
+@pytest.mark.parametrize("norm,distribute", [(0, False), (1, True)])
+def test_blocked_sweeps_match_oracle(oracle_mod, rmat, norm, distribute):
+    csr, dg = rmat
+    tol = 1e-10 if norm == 0 else 1e-12
+    o = oracle_mod.pagerank(csr, tol=tol, norm=norm, distribute_sinks=distribute, nthreads=THREADS)
+    p = dg.params(0.85, tol, norm, False, distribute, _capi.NKG_PREC_FP64, _capi.UINT64_MAX)
+    s, it, _, _ = dg.run(p)
+    assert abs(it - o.iterations) <= 1
+    assert np.abs(s - o.scores).sum() <= 1e-10
+    s2, it2, _, _ = dg.run(p)
+    np.testing.assert_array_equal(s, s2)
+    assert it == it2
+    if norm == 0:
+        p = dg.params(0.85, tol, norm, False, distribute, _capi.NKG_PREC_FP32_REFINE, 10000)
+        s, _, _, _ = dg.run(p)
+        # both stop at a residual of 1e-10, at most 1e-10 / (1 - 0.85) from the fixed point
+        assert np.abs(s - o.scores).sum() <= 2e-9
+
+
+def test_blocked_centralities_match_oracle(oracle_mod, rmat):
+    csr, dg = rmat
+    s, it, _ = dg.eigenvector(1e-9)
+    o, _ = oracle_mod.eigenvector(csr, -1.0, max_iterations=it)
+    assert np.abs(s - o).sum() <= 1e-10 * np.abs(o).sum()
+    s, it, _ = dg.katz(0.0, 0.1, 1e-8, 0)
+    o, _ = oracle_mod.katz(csr.z, csr.in_ptr, csr.in_col, alpha=0.0, beta=0.1, tol=-1.0,
+                           max_degree=int(csr.outdeg.max()), max_iterations=it)
+    # scores of unit 2-norm over 2^22 nodes: L1 up to 2048
+    assert np.abs(s - o).sum() <= 1e-10 * np.abs(o).sum()
+
+
+def test_blocked_ppr_columns_match_the_fp64_run(rmat):
+    csr, dg = rmat
+    seeds = np.array([5, 1 << 21, 77], np.uint32)
+    p = dg.params(0.85, 1e-8, 0, False, True, _capi.NKG_PREC_FP32, 300)
+    got, _, _ = dg.ppr(seeds, p)
+    p64 = dg.params(0.85, 1e-12, 0, False, True, _capi.NKG_PREC_FP64, 2000)
+    for j, u in enumerate(seeds):
+        t = np.zeros(csr.z)
+        t[u] = 1.0
+        assert np.abs(got[j] - dg.run(p64, t)[0]).sum() <= 1e-6
+
+
+def test_blocked_weights_and_gradients(oracle_mod, rmat):
+    a = generators.with_uniform_weights(rmat[0], seed=3)
+    b = generators.with_uniform_weights(rmat[0], seed=4)
+    dg, ref = _capi.DeviceGraph(a), _capi.DeviceGraph(b)
+    p = dg.params(0.85, 1e-10, 0, False, True, _capi.NKG_PREC_FP64, 500)
+    dg.run(p)
+    dg.set_weights(b.in_w, b.wdeg)
+    got, want = dg.run(p)[0], ref.run(p)[0]
+    np.testing.assert_array_equal(got, want)
+    o = oracle_mod.pagerank(b, tol=1e-10, norm=0, distribute_sinks=True, nthreads=THREADS)
+    assert np.abs(want - o.scores).sum() <= 1e-10
+    g = np.random.default_rng(0).standard_normal(a.z)
+    bwd = dg.params(0.85, 1e-11, 0, False, True, _capi.NKG_PREC_FP32_REFINE, _capi.UINT64_MAX)
+    b64 = dg.params(0.85, 1e-12, 0, False, True, _capi.NKG_PREC_FP64, _capi.UINT64_MAX)
+    gw, gt, _, _ = dg.adjoint(bwd, want, g)
+    gw2, gt2, _, _ = ref.adjoint(b64, want, g)
+    assert np.abs(gw - gw2).max() <= 1e-9 * np.abs(gw2).max()
+    assert np.abs(gt - gt2).max() <= 1e-9 * np.abs(gt2).max()
+    # central differences of the FP64 forward on the arcs of the largest gradients
+    for e in np.argsort(-np.abs(gw2))[[0, 3]]:
+        vals = []
+        for h in (1e-4, -1e-4):
+            w = b.in_w.copy()
+            w[e] += h
+            dg.set_weights(w)
+            vals.append(float(g @ dg.run(dg.params(0.85, 0.0, 0, False, True, 0, 250))[0]))
+        fd = (vals[0] - vals[1]) / 2e-4
+        assert abs(fd - gw2[e]) <= 1e-4 * abs(gw2[e])
