@@ -4,12 +4,16 @@
 // t_j). Per column: FP64 residual, FP64 sink mass, and the column stops
 // (freezes) once its residual is at most tol.
 //
-// Layout: the iterate is node-major, Y[r * kp + j] (kp = 32 * CPL columns,
-// CPL per lane), in gather form (x/deg, sinks x). A warp owns one virtual
-// row (a whole row, or a kChunk-arc chunk of a long row); per arc it broadcasts
-// the source id and every lane loads its CPL columns of that source's row:
-// kp * 4 contiguous bytes per arc, float4-coalesced. Warps walk contiguous,
-// cost-balanced ranges of virtual rows, so every sum has a fixed order.
+// Layout: the iterate is node-major, Y[r * kp + j], in gather form (x/deg,
+// sinks x), with kp the columns rounded up to whole 32-byte sectors (k = 37:
+// 40 columns, where rows padded to 128 columns moved 3.2 times the bytes).
+// A virtual row is a whole row, or a kChunk-arc chunk of a long row; warps
+// walk contiguous, cost-balanced ranges of them, so every sum has a fixed
+// order. Up to 128 columns (ppr_sweep) a lane holds 4 columns of a row and the
+// warp's groups of `lanes` lanes take different arcs of the same row (37
+// columns: 3 arcs at a time); the groups' sums are added at the row's end. Rows of more than 128 columns
+// (ppr_sweep_bulk) come as bulk copies through shared memory. The other kernels treat a row of
+// more than 128 columns as two parts, each the work of its own warp.
 #include <cub/cub.cuh>
 
 #include <algorithm>
@@ -25,11 +29,14 @@ namespace {
 
 constexpr int kPprThreads = 256;
 constexpr int kPprWarps = kPprThreads / 32;
+constexpr uint32_t kPprBatch = 4;  // arcs of a lane in flight (6 and 8 cost warps: slower)
 
 struct PprState {
     unsigned long long iteration;
     int all_done;
     unsigned int ticket;
+    int error;  // a bulk copy did not arrive
+    int pad;
 };
 
 struct PprArgs {
@@ -37,7 +44,7 @@ struct PprArgs {
     const uint32_t *__restrict__ col;
     const uint32_t *__restrict__ degc;
     const uint32_t *__restrict__ chunk_begin;  // n_long+1
-    const uint32_t *__restrict__ chunk_row;    // per chunk: its row
+    const uint2 *__restrict__ vrange;          // per virtual row: its arcs [x, y)
     const uint32_t *__restrict__ unit_start;   // units+1 virtual-row indices
     const uint32_t *__restrict__ seed;         // kp: relabelled seed id (kNone: padding column)
     const float *__restrict__ y_in;            // n * kp
@@ -53,230 +60,456 @@ struct PprArgs {
     double damp, tol;
     unsigned long long max_iterations;
     uint32_t n, n_long, n_chunks, units, kp, sweep_ctas;
+    uint32_t lanes, groups, parts;             // lane layout of a row (above)
     int l2, distribute;
 };
 
-// Virtual rows: [0, n_chunks) chunks of the long rows, then rows n_long..n-1.
-__device__ __forceinline__ void vrow_range(const PprArgs &a, uint32_t v, uint32_t &r, uint32_t &b,
-                                           uint32_t &e) {
-    if (v < a.n_chunks) {
-        r = a.chunk_row[v];
-        const uint32_t c = v - a.chunk_begin[r];
-        b = a.row_ptr[r] + c * kChunk;
-        e = min(a.row_ptr[r + 1], b + kChunk);
-    } else {
-        r = a.n_long + (v - a.n_chunks);
-        b = a.row_ptr[r];
-        e = a.row_ptr[r + 1];
-    }
+// This lane's place in the layout: its group of lanes (>= groups: idle), its
+// first column, whether it finishes rows (group 0).
+struct PprLane {
+    uint32_t group, col;
+    bool on;     // loads columns
+    bool first;  // holds the row's sums
+};
+__device__ __forceinline__ PprLane ppr_lane(const PprArgs &a) {
+    const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    PprLane L;
+    L.group = lane / a.lanes;
+    L.on = L.group < a.groups;
+    L.first = L.group == 0;
+    L.col = ((wid & (a.parts - 1)) * a.lanes + lane % a.lanes) * 4;
+    return L;
 }
 
-template <int CPL>
-__device__ __forceinline__ void accumulate(const PprArgs &a, uint32_t b, uint32_t e, int lane,
-                                           float (&acc)[CPL]) {
+// Virtual rows: [0, n_chunks) chunks of the long rows, then rows n_long..n-1.
+
+__device__ __forceinline__ void add4(float (&acc)[4], const float4 &v) {
+    acc[0] += v.x;
+    acc[1] += v.y;
+    acc[2] += v.z;
+    acc[3] += v.w;
+}
+
+// Sum of the source rows of arcs [b, e) in this lane's columns. Group g takes
+// arcs g, g + groups, ...; the groups' sums are added into group 0, in group
+// order.
+__device__ __forceinline__ void accumulate(const PprArgs &a, const PprLane &L, uint32_t b,
+                                           uint32_t e, float (&acc)[4]) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t groups = a.groups;
+    const float *y = a.y_in + L.col;
 #pragma unroll
-    for (int q = 0; q < CPL; ++q)
-        acc[q] = 0.f;
+    for (int c = 0; c < 4; ++c)
+        acc[c] = 0.f;
     for (uint32_t base = b; base < e; base += 32) {
         const uint32_t cnt = min(32u, e - base);
-        const uint32_t cl = lane < static_cast<int>(cnt) ? ld_stream(a.col + base + lane) : 0u;
-        uint32_t i = 0;
-        for (; i + 4 <= cnt; i += 4) {
-            float4 v[4][CPL / 4];
+        const uint32_t cl = lane < cnt ? ld_stream(a.col + base + lane) : 0u;
+        for (uint32_t i = 0; i < cnt; i += kPprBatch * groups) {
+            float4 v[kPprBatch];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const uint32_t src = __shfl_sync(0xffffffffu, cl, i + u);
-                const float4 *p =
-                    reinterpret_cast<const float4 *>(a.y_in + static_cast<size_t>(src) * a.kp) +
-                    lane * (CPL / 4);
-#pragma unroll
-                for (int q = 0; q < CPL / 4; ++q)
-                    v[u][q] = __ldg(p + q);
+            for (uint32_t u = 0; u < kPprBatch; ++u) {
+                const uint32_t k = i + u * groups + L.group;
+                const uint32_t src = __shfl_sync(0xffffffffu, cl, k & 31);
+                v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (L.on && k < cnt)
+                    v[u] = __ldg(reinterpret_cast<const float4 *>(y + static_cast<size_t>(src) * a.kp));
             }
 #pragma unroll
-            for (int u = 0; u < 4; ++u)
-#pragma unroll
-                for (int q = 0; q < CPL / 4; ++q) {
-                    acc[4 * q + 0] += v[u][q].x;
-                    acc[4 * q + 1] += v[u][q].y;
-                    acc[4 * q + 2] += v[u][q].z;
-                    acc[4 * q + 3] += v[u][q].w;
-                }
+            for (uint32_t u = 0; u < kPprBatch; ++u)
+                add4(acc, v[u]);
         }
-        for (; i < cnt; ++i) {
-            const uint32_t src = __shfl_sync(0xffffffffu, cl, i);
-            const float4 *p =
-                reinterpret_cast<const float4 *>(a.y_in + static_cast<size_t>(src) * a.kp) +
-                lane * (CPL / 4);
+    }
+    const float t[4] = {acc[0], acc[1], acc[2], acc[3]};
+    for (uint32_t g = 1; g < groups; ++g) {
 #pragma unroll
-            for (int q = 0; q < CPL / 4; ++q) {
-                const float4 v = __ldg(p + q);
-                acc[4 * q + 0] += v.x;
-                acc[4 * q + 1] += v.y;
-                acc[4 * q + 2] += v.z;
-                acc[4 * q + 3] += v.w;
-            }
-        }
+        for (int c = 0; c < 4; ++c)
+            acc[c] += __shfl_sync(0xffffffffu, t[c], (lane + g * a.lanes) & 31);
     }
 }
 
-// Finish row r for this lane's CPL columns.
-template <int CPL>
-__device__ __forceinline__ void finish(const PprArgs &a, uint32_t r, int lane, const float (&acc)[CPL],
-                                       const int (&act)[CPL], const float (&sc)[CPL],
-                                       const uint32_t (&seed)[CPL], double (&res)[CPL],
-                                       double (&sink)[CPL]) {
+// Row r's new value in one column (PageRank.cpp:64-65 in gather form) from its
+// sum; frozen columns keep the old one.
+__device__ __forceinline__ float finish_column(const PprArgs &a, uint32_t r, uint32_t dc, float deg,
+                                               float dampf, float omd, float sum, float yo, int act,
+                                               float sc, uint32_t seed, double &res, double &sink) {
+    if (!act)
+        return yo;
+    const float tel = (r == seed) ? 1.f : 0.f;
+    if (a.distribute)
+        sum = __fadd_rn(sum, __fmul_rn(sc, tel));
+    float x = __fmul_rn(sum, dampf);
+    x = __fadd_rn(x, __fmul_rn(omd, tel));
+    const float xo = dc ? __fmul_rn(yo, deg) : yo;
+    const double d = static_cast<double>(xo) - static_cast<double>(x);
+    res += a.l2 ? d * d : fabs(d);
+    if (dc)
+        return x / deg;
+    sink += static_cast<double>(x);
+    return x;
+}
+
+// Finish row r for this lane's columns. What is constant per column is loaded
+// here: held across the gathers it made the sweep spill at 64 registers.
+__device__ __forceinline__ void finish(const PprArgs &a, const PprLane &L, uint32_t r,
+                                       const float (&acc)[4], double (&res)[4], double (&sink)[4]) {
+    const int4 on = __ldg(reinterpret_cast<const int4 *>(a.active + L.col));
+    const uint4 sd = __ldg(reinterpret_cast<const uint4 *>(a.seed + L.col));
+    const float4 s4 = a.distribute ? __ldg(reinterpret_cast<const float4 *>(a.sink_coef + L.col))
+                                   : make_float4(0.f, 0.f, 0.f, 0.f);
+    const int act[4] = {on.x, on.y, on.z, on.w};
+    const uint32_t seed[4] = {sd.x, sd.y, sd.z, sd.w};
+    const float sc[4] = {s4.x, s4.y, s4.z, s4.w};
     const uint32_t dc = ld_stream(a.degc + r);
     const float deg = static_cast<float>(dc);
-    const float4 *pin = reinterpret_cast<const float4 *>(a.y_in + static_cast<size_t>(r) * a.kp) +
-                        lane * (CPL / 4);
-    float4 *pout = reinterpret_cast<float4 *>(a.y_out + static_cast<size_t>(r) * a.kp) +
-                   lane * (CPL / 4);
+    const size_t at = static_cast<size_t>(r) * a.kp + L.col;
     const float dampf = static_cast<float>(a.damp), omd = static_cast<float>(1.0 - a.damp);
+    const float4 yo4 = __ldg(reinterpret_cast<const float4 *>(a.y_in + at));
+    const float yo[4] = {yo4.x, yo4.y, yo4.z, yo4.w};
+    float yn[4];
 #pragma unroll
-    for (int q = 0; q < CPL / 4; ++q) {
-        const float4 yo4 = __ldg(pin + q);
-        float yo[4] = {yo4.x, yo4.y, yo4.z, yo4.w};
-        float yn[4];
-#pragma unroll
-        for (int t = 0; t < 4; ++t) {
-            const int c = 4 * q + t;
-            if (!act[c]) {
-                yn[t] = yo[t];
-                continue;
-            }
-            const float tel = (r == seed[c]) ? 1.f : 0.f;
-            float s = acc[c];
-            if (a.distribute)
-                s = __fadd_rn(s, __fmul_rn(sc[c], tel));
-            float x = __fmul_rn(s, dampf);
-            x = __fadd_rn(x, __fmul_rn(omd, tel));
-            const float xo = dc ? __fmul_rn(yo[t], deg) : yo[t];
-            const double d = static_cast<double>(xo) - static_cast<double>(x);
-            res[c] += a.l2 ? d * d : fabs(d);
-            if (dc) {
-                yn[t] = x / deg;
-            } else {
-                yn[t] = x;
-                sink[c] += static_cast<double>(x);
-            }
-        }
-        pout[q] = make_float4(yn[0], yn[1], yn[2], yn[3]);
-    }
+    for (int c = 0; c < 4; ++c)
+        yn[c] = finish_column(a, r, dc, deg, dampf, omd, acc[c], yo[c], act[c], sc[c], seed[c],
+                              res[c], sink[c]);
+    *reinterpret_cast<float4 *>(a.y_out + at) = make_float4(yn[0], yn[1], yn[2], yn[3]);
 }
 
-// Per-column block reduction of res/sink into cta_res/cta_sink[blockIdx.x*kp ..].
-template <int CPL>
-__device__ __forceinline__ void column_partials(const PprArgs &a, int lane, const double (&res)[CPL],
-                                                const double (&sink)[CPL], double *s_buf,
-                                                double *out_res, double *out_sink) {
-    const int wid = threadIdx.x >> 5;
-    const uint32_t kp = a.kp;
+// Per-column block sums of `res` and `sink` over the warps (and, with `groups`
+// > 1, the groups of lanes) that hold the column, plus rows blockIdx.x,
+// blockIdx.x + gridDim.x, ... of `more` rows of earlier partials, into
+// out_res/out_sink[blockIdx.x * kp ..]. s_buf: kPprWarps * 128 doubles.
+__device__ __forceinline__ void column_partials(const PprArgs &a, const PprLane &L, uint32_t groups,
+                                                const double (&res)[4], const double (&sink)[4],
+                                                double *s_buf, double *out_res, double *out_sink,
+                                                const double *more_res, const double *more_sink,
+                                                uint32_t more) {
+    const uint32_t wid = threadIdx.x >> 5, kp = a.kp, w4 = 4 * a.lanes;
+    const uint32_t part_col = L.col - (wid & (a.parts - 1)) * w4;
     for (int pass = 0; pass < 2; ++pass) {
         __syncthreads();
+        if (L.group < groups)
 #pragma unroll
-        for (int c = 0; c < CPL; ++c)
-            s_buf[wid * kp + lane * CPL + c] = pass == 0 ? res[c] : sink[c];
+            for (int c = 0; c < 4; ++c)
+                s_buf[(wid * groups + L.group) * w4 + part_col + c] = pass == 0 ? res[c] : sink[c];
         __syncthreads();
+        const double *m = pass == 0 ? more_res : more_sink;
         for (uint32_t col = threadIdx.x; col < kp; col += kPprThreads) {
+            const uint32_t part = col / w4;
             double s = 0.0;
-            for (int w = 0; w < kPprWarps; ++w)
-                s += s_buf[w * kp + col];
+            for (uint32_t w = part; w < kPprWarps; w += a.parts)
+                for (uint32_t g = 0; g < groups; ++g)
+                    s += s_buf[(w * groups + g) * w4 + col - part * w4];
+#pragma unroll 4
+            for (uint32_t i = blockIdx.x; i < more; i += gridDim.x)
+                s += m[static_cast<size_t>(i) * kp + col];
             (pass == 0 ? out_res : out_sink)[static_cast<size_t>(blockIdx.x) * kp + col] = s;
         }
     }
     __threadfence();  // partials visible device-wide before any ticket
 }
 
-template <int CPL>
-__device__ __forceinline__ void load_columns(const PprArgs &a, int lane, int (&act)[CPL],
-                                             float (&sc)[CPL], uint32_t (&seed)[CPL]) {
+// ---------------------------------------------------------------------------
+// The sweep of wide rows (more than 128 columns): the rows of a unit's arcs
+// are bulk copies into a ring of shared memory per warp, issued along the
+// arcs of the unit without regard to row bounds, so that about 190 KB per SM
+// are in flight all the time. With the rows loaded into registers (4 arcs of
+// 1 KB per warp, 16 warps per SM) every row's end left the warp with nothing
+// in flight for two dependent loads.
+constexpr int kBulkWarps = 16;
+constexpr int kBulkThreads = kBulkWarps * 32;
+constexpr uint32_t kBulkArcs = 4;        // arcs per stage
+constexpr uint32_t kBulkStages = 8;      // most stages of a warp's ring
+constexpr uint32_t kBulkPolls = 1u << 20;  // a wait gives up after about a second
+constexpr size_t kBulkBytes = 216 * 1024;
+
+__device__ __forceinline__ uint32_t smem_addr(const void *p) {
+    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
+}
+__device__ __forceinline__ void bar_init(uint64_t *b) {
+    asm volatile("mbarrier.init.shared.b64 [%0], 1;" ::"r"(smem_addr(b)) : "memory");
+}
+__device__ __forceinline__ void bar_expect(uint64_t *b, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared.b64 _, [%0], %1;" ::"r"(smem_addr(b)), "r"(bytes)
+                 : "memory");
+}
+// True once the phase is complete; false when the wait ran out.
+__device__ __forceinline__ bool bar_wait(uint64_t *b, uint32_t phase) {
+    for (uint32_t i = 0; i < kBulkPolls; ++i) {
+        uint32_t ok;
+        asm volatile("{\n .reg .pred p;\n"
+                     " mbarrier.try_wait.parity.shared.b64 p, [%1], %2;\n"
+                     " selp.u32 %0, 1, 0, p;\n}"
+                     : "=r"(ok)
+                     : "r"(smem_addr(b)), "r"(phase)
+                     : "memory");
+        if (ok)
+            return true;
+    }
+    return false;
+}
+__device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t bytes, uint64_t *b) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 ::"r"(smem_addr(dst)), "l"(src), "r"(bytes), "r"(smem_addr(b))
+                 : "memory");
+}
+
+// One warp's ring over the arcs [next, end): stages of kBulkArcs rows.
+struct PprRing {
+    unsigned char *rows;  // the warp's stages
+    uint64_t *bar;
+    uint32_t stages, row_bytes;
+    uint32_t begin, next, end;  // next arc to issue
+    uint32_t window;            // sources of the 32 arcs the next one lies in
+    uint32_t fill, phases;      // stage to fill; parity of every stage's next wait
+};
+
+__device__ __forceinline__ void ring_issue(const PprArgs &a, PprRing &q) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t n = min(kBulkArcs, q.end - q.next);
+    if (!n)
+        return;
+    const uint32_t at = (q.next - q.begin) & 31;
+    if (at == 0)
+        q.window = q.next + lane < q.end ? ld_stream(a.col + q.next + lane) : 0u;
+    const uint32_t src = __shfl_sync(0xffffffffu, q.window, (at + lane) & 31);
+    if (lane == 0)
+        bar_expect(q.bar + q.fill, n * q.row_bytes);
+    __syncwarp();
+    if (lane < n)
+        bulk_load(q.rows + (q.fill * kBulkArcs + lane) * q.row_bytes,
+                  a.y_in + static_cast<size_t>(src) * a.kp, q.row_bytes, q.bar + q.fill);
+    q.next += n;
+    q.fill = q.fill + 1 == q.stages ? 0 : q.fill + 1;
+}
+
+// A lane holds columns h * 128 + 4 lane ..+3 for h = 0, 1.
+__global__ void __launch_bounds__(kBulkThreads, 1) ppr_sweep_bulk(PprArgs a, uint32_t stages) {
+    constexpr int H = 2;
+    extern __shared__ __align__(128) unsigned char s_ring[];
+    __shared__ uint64_t s_bar[kBulkWarps][kBulkStages];
+    if (*(volatile int *)&a.st->all_done)
+        return;
+    const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    if (lane == 0)
+        for (uint32_t i = 0; i < stages; ++i)
+            bar_init(&s_bar[wid][i]);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async;" ::: "memory");
+    __syncwarp();
+    const float dampf = static_cast<float>(a.damp), omd = static_cast<float>(1.0 - a.damp);
+    bool on[H];
+    int act[H][4];
+    float sc[H][4];
+    uint32_t seed[H][4];
+    double res[H][4], sink[H][4];
 #pragma unroll
-    for (int c = 0; c < CPL; ++c) {
-        const uint32_t col = lane * CPL + c;
-        act[c] = a.active[col];
-        sc[c] = a.sink_coef[col];
-        seed[c] = a.seed[col];
+    for (int h = 0; h < H; ++h) {
+        const uint32_t c0 = h * 128 + lane * 4;
+        on[h] = c0 < a.kp;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            act[h][c] = on[h] ? a.active[c0 + c] : 0;
+            sc[h][c] = on[h] ? a.sink_coef[c0 + c] : 0.f;
+            seed[h][c] = on[h] ? a.seed[c0 + c] : kNone;
+            res[h][c] = sink[h][c] = 0.0;
+        }
+    }
+    PprRing q;
+    q.row_bytes = a.kp * 4;
+    q.stages = stages;
+    q.rows = s_ring + static_cast<size_t>(wid) * stages * kBulkArcs * q.row_bytes;
+    q.bar = s_bar[wid];
+    q.fill = 0;
+    q.phases = 0;
+    q.window = 0;
+    uint32_t cur = 0;  // stage to read next
+    bool ok = true;
+    const uint32_t gw = blockIdx.x * kBulkWarps + wid, nw = gridDim.x * kBulkWarps;
+    for (uint32_t u = gw; u < a.units && ok; u += nw) {
+        const uint32_t v_end = a.unit_start[u + 1];
+        uint32_t v = a.unit_start[u];
+        if (v >= v_end)
+            continue;
+        q.begin = q.next = __ldg(a.vrange + v).x;
+        q.end = __ldg(a.vrange + v_end - 1).y;
+        for (uint32_t i = 0; i < stages; ++i)
+            ring_issue(a, q);
+        uint32_t k = q.begin;
+        uint32_t e = __ldg(a.vrange + v).y;
+        float acc[H][4];
+        float4 yo[H];
+        uint32_t dc = 0;
+        // Row v's own entries, wanted at its end, are loaded at its start.
+        auto open_row = [&]() {
+#pragma unroll
+            for (int h = 0; h < H; ++h) {
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+                    acc[h][c] = 0.f;
+                yo[h] = make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+            if (v >= a.n_chunks) {
+                const uint32_t r = a.n_long + (v - a.n_chunks);
+                dc = ld_stream(a.degc + r);
+#pragma unroll
+                for (int h = 0; h < H; ++h)
+                    if (on[h])
+                        yo[h] = __ldg(reinterpret_cast<const float4 *>(
+                            a.y_in + static_cast<size_t>(r) * a.kp + h * 128 + lane * 4));
+            }
+        };
+        auto close_row = [&]() {
+            if (v < a.n_chunks) {
+#pragma unroll
+                for (int h = 0; h < H; ++h)
+                    if (on[h])
+                        *reinterpret_cast<float4 *>(a.chunk_val + static_cast<size_t>(v) * a.kp +
+                                                    h * 128 + lane * 4) =
+                            make_float4(acc[h][0], acc[h][1], acc[h][2], acc[h][3]);
+                return;
+            }
+            const uint32_t r = a.n_long + (v - a.n_chunks);
+            const float deg = static_cast<float>(dc);
+#pragma unroll
+            for (int h = 0; h < H; ++h) {
+                const float y[4] = {yo[h].x, yo[h].y, yo[h].z, yo[h].w};
+                float yn[4];
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+                    yn[c] = finish_column(a, r, dc, deg, dampf, omd, acc[h][c], y[c], act[h][c],
+                                          sc[h][c], seed[h][c], res[h][c], sink[h][c]);
+                if (on[h])
+                    *reinterpret_cast<float4 *>(a.y_out + static_cast<size_t>(r) * a.kp + h * 128 +
+                                                lane * 4) = make_float4(yn[0], yn[1], yn[2], yn[3]);
+            }
+        };
+        open_row();
+        while (k < q.end) {
+            if (!bar_wait(q.bar + cur, (q.phases >> cur) & 1)) {
+                ok = false;
+                break;
+            }
+            q.phases ^= 1u << cur;
+            const uint32_t n = min(kBulkArcs, q.end - k);
+            const unsigned char *st = q.rows + cur * kBulkArcs * q.row_bytes + lane * 16;
+            for (uint32_t i = 0; i < n; ++i, ++k) {
+                while (k == e) {
+                    close_row();
+                    ++v;
+                    e = __ldg(a.vrange + v).y;
+                    open_row();
+                }
+#pragma unroll
+                for (int h = 0; h < H; ++h)
+                    if (on[h])
+                        add4(acc[h], *reinterpret_cast<const float4 *>(st + i * q.row_bytes + h * 512));
+            }
+            __syncwarp();  // every lane has read the stage
+            cur = cur + 1 == stages ? 0 : cur + 1;
+            ring_issue(a, q);
+        }
+        if (!ok)
+            break;
+        for (;;) {  // the last row with arcs and the empty rows behind it
+            close_row();
+            if (++v >= v_end)
+                break;
+            open_row();
+        }
+    }
+    if (!ok) {
+        // A copy never arrived: report it, and give the others their time.
+        if (lane == 0)
+            a.st->error = 1;
+        for (uint32_t i = 0; i < stages; ++i)
+            bar_wait(q.bar + i, (q.phases >> i) & 1);
+    }
+    // Per-column sums over the warps (column_partials).
+    double *s_buf = reinterpret_cast<double *>(s_ring);
+    for (int pass = 0; pass < 2; ++pass) {
+        __syncthreads();
+#pragma unroll
+        for (int h = 0; h < H; ++h)
+            if (on[h])
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+                    s_buf[wid * a.kp + h * 128 + lane * 4 + c] = pass == 0 ? res[h][c] : sink[h][c];
+        __syncthreads();
+        for (uint32_t col = threadIdx.x; col < a.kp; col += kBulkThreads) {
+            double sum = 0.0;
+            for (uint32_t w = 0; w < kBulkWarps; ++w)
+                sum += s_buf[w * a.kp + col];
+            (pass == 0 ? a.cta_res : a.cta_sink)[static_cast<size_t>(blockIdx.x) * a.kp + col] = sum;
+        }
     }
 }
 
-template <int CPL>
-__global__ void __launch_bounds__(kPprThreads) ppr_sweep(PprArgs a) {
+__global__ void __launch_bounds__(kPprThreads, 4) ppr_sweep(PprArgs a) {
     extern __shared__ double s_buf[];
     if (*(volatile int *)&a.st->all_done)
         return;
-    const int lane = threadIdx.x & 31;
-    int act[CPL];
-    float sc[CPL];
-    uint32_t seed[CPL];
-    load_columns<CPL>(a, lane, act, sc, seed);
-    double res[CPL], sink[CPL];
+    const uint32_t lane = threadIdx.x & 31;
+    const PprLane L = ppr_lane(a);
+    double res[4], sink[4];
 #pragma unroll
-    for (int c = 0; c < CPL; ++c)
+    for (int c = 0; c < 4; ++c)
         res[c] = sink[c] = 0.0;
     const uint32_t gw = blockIdx.x * kPprWarps + (threadIdx.x >> 5);
     const uint32_t nw = gridDim.x * kPprWarps;
     for (uint32_t u = gw; u < a.units; u += nw) {
         const uint32_t v_end = a.unit_start[u + 1];
-        for (uint32_t v = a.unit_start[u]; v < v_end; ++v) {
-            uint32_t r, b, e;
-            vrow_range(a, v, r, b, e);
-            float acc[CPL];
-            accumulate<CPL>(a, b, e, lane, acc);
-            if (v < a.n_chunks) {
-                float4 *p = reinterpret_cast<float4 *>(a.chunk_val + static_cast<size_t>(v) * a.kp) +
-                            lane * (CPL / 4);
-#pragma unroll
-                for (int q = 0; q < CPL / 4; ++q)
-                    p[q] = make_float4(acc[4 * q], acc[4 * q + 1], acc[4 * q + 2], acc[4 * q + 3]);
-            } else {
-                finish<CPL>(a, r, lane, acc, act, sc, seed, res, sink);
+        uint32_t v = a.unit_start[u];
+        if (v >= v_end)
+            continue;
+        uint2 cur = __ldg(a.vrange + v);
+        for (; v < v_end; ++v) {
+            const uint2 nxt = v + 1 < v_end ? __ldg(a.vrange + v + 1) : make_uint2(0u, 0u);
+            float acc[4];
+            accumulate(a, L, cur.x, cur.y, acc);
+            if (L.first) {
+                if (v < a.n_chunks)
+                    *reinterpret_cast<float4 *>(a.chunk_val + static_cast<size_t>(v) * a.kp + L.col) =
+                        make_float4(acc[0], acc[1], acc[2], acc[3]);
+                else
+                    finish(a, L, a.n_long + (v - a.n_chunks), acc, res, sink);
             }
+            cur = nxt;
         }
     }
-    column_partials<CPL>(a, lane, res, sink, s_buf, a.cta_res, a.cta_sink);
+    column_partials(a, L, 1, res, sink, s_buf, a.cta_res, a.cta_sink, nullptr, nullptr, 0);
 }
 
-// Long rows: sum their chunk partials in order (one warp per row), finish
-// them, then the last CTA closes the iteration per column.
-template <int CPL>
+// Long rows: sum their chunk partials in order (a warp per row and part),
+// finish them, then the last CTA closes the iteration per column. Every CTA
+// adds its share of the sweep's per-CTA partials to its own, so the last one
+// is left with gridDim.x rows of partials, which it adds eight at a time (one
+// CTA that added the sweep's 600 to 900 rows itself, one after the other, took
+// 0.4 ms of every sweep).
 __global__ void __launch_bounds__(kPprThreads) ppr_fixup(PprArgs a, double *fix_res,
                                                          double *fix_sink) {
     extern __shared__ double s_buf[];
     __shared__ bool s_last;
     if (*(volatile int *)&a.st->all_done)
         return;
-    const int lane = threadIdx.x & 31;
-    int act[CPL];
-    float sc[CPL];
-    uint32_t seed[CPL];
-    load_columns<CPL>(a, lane, act, sc, seed);
-    double res[CPL], sink[CPL];
+    const PprLane L = ppr_lane(a);
+    double res[4], sink[4];
 #pragma unroll
-    for (int c = 0; c < CPL; ++c)
+    for (int c = 0; c < 4; ++c)
         res[c] = sink[c] = 0.0;
-    const uint32_t gw = blockIdx.x * kPprWarps + (threadIdx.x >> 5);
-    const uint32_t nw = gridDim.x * kPprWarps;
+    const uint32_t wpc = kPprWarps / a.parts;
+    const uint32_t gw = blockIdx.x * wpc + (threadIdx.x >> 5) / a.parts;
+    const uint32_t nw = gridDim.x * wpc;
     for (uint32_t r = gw; r < a.n_long; r += nw) {
-        float acc[CPL];
-#pragma unroll
-        for (int c = 0; c < CPL; ++c)
-            acc[c] = 0.f;
-        for (uint32_t k = a.chunk_begin[r]; k < a.chunk_begin[r + 1]; ++k) {
-            const float4 *p = reinterpret_cast<const float4 *>(a.chunk_val + static_cast<size_t>(k) * a.kp) +
-                              lane * (CPL / 4);
-#pragma unroll
-            for (int q = 0; q < CPL / 4; ++q) {
-                const float4 v = p[q];
-                acc[4 * q] += v.x;
-                acc[4 * q + 1] += v.y;
-                acc[4 * q + 2] += v.z;
-                acc[4 * q + 3] += v.w;
-            }
-        }
-        finish<CPL>(a, r, lane, acc, act, sc, seed, res, sink);
+        if (!L.first)
+            continue;
+        float acc[4] = {0.f, 0.f, 0.f, 0.f};
+        const uint32_t ke = a.chunk_begin[r + 1];
+#pragma unroll 8
+        for (uint32_t k = a.chunk_begin[r]; k < ke; ++k)
+            add4(acc, *reinterpret_cast<const float4 *>(a.chunk_val + static_cast<size_t>(k) * a.kp + L.col));
+        finish(a, L, r, acc, res, sink);
     }
-    column_partials<CPL>(a, lane, res, sink, s_buf, fix_res, fix_sink);
+    column_partials(a, L, 1, res, sink, s_buf, fix_res, fix_sink, a.cta_res, a.cta_sink,
+                    a.sweep_ctas);
     __syncthreads();
     if (threadIdx.x == 0) {
         __threadfence();
@@ -290,13 +523,10 @@ __global__ void __launch_bounds__(kPprThreads) ppr_fixup(PprArgs a, double *fix_
     int any_active = 0;
     for (uint32_t col = threadIdx.x; col < a.kp; col += kPprThreads) {
         double r = 0.0, s = 0.0;
-        for (uint32_t i = 0; i < a.sweep_ctas; ++i) {
-            r += ((volatile double *)a.cta_res)[static_cast<size_t>(i) * a.kp + col];
-            s += ((volatile double *)a.cta_sink)[static_cast<size_t>(i) * a.kp + col];
-        }
+#pragma unroll 8
         for (uint32_t i = 0; i < gridDim.x; ++i) {
-            r += ((volatile double *)fix_res)[static_cast<size_t>(i) * a.kp + col];
-            s += ((volatile double *)fix_sink)[static_cast<size_t>(i) * a.kp + col];
+            r += __ldcg(fix_res + static_cast<size_t>(i) * a.kp + col);
+            s += __ldcg(fix_sink + static_cast<size_t>(i) * a.kp + col);
         }
         if (a.active[col]) {
             const double norm = a.l2 ? sqrt(r) : r;
@@ -328,38 +558,36 @@ __global__ void ppr_init(float *__restrict__ y, const uint32_t *__restrict__ deg
     y[i] = dc ? x0 / static_cast<float>(dc) : x0;
 }
 
-// Column sums of x (and of x over sinks), FP64, fixed order: one warp per row.
-template <int CPL>
-__global__ void __launch_bounds__(kPprThreads) ppr_colsum(const float *__restrict__ y,
-                                                          const uint32_t *__restrict__ degc,
-                                                          uint32_t n, uint32_t kp, double *part_sum,
-                                                          double *part_sink) {
+// Column sums of x (and of x over sinks), FP64, fixed order: every group of
+// lanes takes rows of its own.
+__global__ void __launch_bounds__(kPprThreads) ppr_colsum(PprArgs a, const float *__restrict__ y,
+                                                          double *part_sum, double *part_sink) {
     extern __shared__ double s_buf[];
-    const int lane = threadIdx.x & 31;
-    double sum[CPL], sink[CPL];
+    const PprLane L = ppr_lane(a);
+    double sum[4], sink[4];
 #pragma unroll
-    for (int c = 0; c < CPL; ++c)
+    for (int c = 0; c < 4; ++c)
         sum[c] = sink[c] = 0.0;
-    for (uint32_t r = blockIdx.x * kPprWarps + (threadIdx.x >> 5); r < n; r += gridDim.x * kPprWarps) {
-        const uint32_t dc = degc[r];
-        const float4 *p = reinterpret_cast<const float4 *>(y + static_cast<size_t>(r) * kp) +
-                          lane * (CPL / 4);
-#pragma unroll
-        for (int q = 0; q < CPL / 4; ++q) {
-            const float4 v = p[q];
+    const uint32_t wpc = kPprWarps / a.parts;
+    const uint32_t gw = blockIdx.x * wpc + (threadIdx.x >> 5) / a.parts;
+    const uint32_t nw = gridDim.x * wpc;
+    if (L.on) {
+#pragma unroll 4
+        for (uint32_t r = gw * a.groups + L.group; r < a.n; r += nw * a.groups) {
+            const uint32_t dc = __ldg(a.degc + r);
+            const float4 v =
+                __ldg(reinterpret_cast<const float4 *>(y + static_cast<size_t>(r) * a.kp + L.col));
             const float vv[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
             for (int t = 0; t < 4; ++t) {
                 const float x = dc ? __fmul_rn(vv[t], static_cast<float>(dc)) : vv[t];
-                sum[4 * q + t] += x;
+                sum[t] += x;
                 if (!dc)
-                    sink[4 * q + t] += x;
+                    sink[t] += x;
             }
         }
     }
-    PprArgs dummy{};
-    dummy.kp = kp;
-    column_partials<CPL>(dummy, lane, sum, sink, s_buf, part_sum, part_sink);
+    column_partials(a, L, a.groups, sum, sink, s_buf, part_sum, part_sink, nullptr, nullptr, 0);
 }
 
 // Column j of the output (caller's ids): out[j*z + o] = x_j(inv[o]) / factor_j.
@@ -396,25 +624,29 @@ __global__ void ppr_output(const float *__restrict__ y, const uint32_t *__restri
     }
 }
 
-__global__ void ppr_vrow_cost(const uint32_t *__restrict__ row_ptr,
-                              const uint32_t *__restrict__ chunk_begin,
-                              const uint32_t *__restrict__ chunk_row, uint32_t n_chunks,
-                              uint32_t n_long, uint32_t n, uint64_t *__restrict__ cost) {
+// Arcs [x, y) and cost of every virtual row.
+__global__ void ppr_vrow_ranges(const uint32_t *__restrict__ row_ptr,
+                                const uint32_t *__restrict__ chunk_begin,
+                                const uint32_t *__restrict__ chunk_row, uint32_t n_chunks,
+                                uint32_t n_long, uint32_t n, uint2 *__restrict__ range,
+                                uint64_t *__restrict__ cost) {
     const uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t nv = n_chunks + (n - n_long);
     if (v >= nv)
         return;
-    uint32_t len;
+    uint32_t b, e;
     if (v < n_chunks) {
         const uint32_t r = chunk_row[v];
         const uint32_t c = v - chunk_begin[r];
-        const uint32_t b = row_ptr[r] + c * kChunk;
-        len = min(row_ptr[r + 1], b + kChunk) - b;
+        b = row_ptr[r] + c * kChunk;
+        e = min(row_ptr[r + 1], b + kChunk);
     } else {
         const uint32_t r = n_long + (v - n_chunks);
-        len = row_ptr[r + 1] - row_ptr[r];
+        b = row_ptr[r];
+        e = row_ptr[r + 1];
     }
-    cost[v] = static_cast<uint64_t>(len) + 4;  // arcs + the row's epilogue
+    range[v] = make_uint2(b, e);
+    cost[v] = static_cast<uint64_t>(e - b) + 4;  // arcs + the row's epilogue
 }
 
 __global__ void ppr_unit_bounds(const uint64_t *__restrict__ cost_incl, uint32_t nv, uint32_t units,
@@ -479,12 +711,17 @@ __global__ void ppr_seeds(const uint32_t *__restrict__ seeds_orig, const uint32_
     }
 }
 
-template <int CPL>
 void run_ppr(nkg_graph *g, const nkg_pr_params &p, uint32_t k, const uint32_t *seeds_host,
              float *out, bool out_on_device, uint64_t *iters_out, nkg_stats *stats) {
     cudaStream_t s = g->stream;
     const uint32_t n = static_cast<uint32_t>(g->n);
-    const uint32_t kp = 32u * CPL;
+    // Lane layout: see the head of this file.
+    const uint32_t parts = k > 128 ? 2 : 1;
+    uint32_t lanes = std::max<uint32_t>(1, ceil_div(k, 4 * parts));
+    if (lanes > 1)
+        lanes = (lanes + 1) / 2 * 2;  // whole 32-byte sectors
+    const uint32_t groups = 32 / lanes;
+    const uint32_t kp = 4 * lanes * parts;
     const unsigned sms = num_sms(g->device);
     NKG_CUDA(cudaEventRecord(g->ev0, s));
 
@@ -504,27 +741,31 @@ void run_ppr(nkg_graph *g, const nkg_pr_params &p, uint32_t k, const uint32_t *s
     if (n_long)
         ppr_chunk_rows<<<sms * 4, 256, 0, s>>>(chunk_begin, n_long, chunk_row.get());
     int occ = 0;
-    const size_t smem_sweep = static_cast<size_t>(kPprWarps) * kp * sizeof(double);
-    NKG_CUDA(cudaFuncSetAttribute(ppr_sweep<CPL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  static_cast<int>(smem_sweep)));
-    NKG_CUDA(cudaFuncSetAttribute(ppr_fixup<CPL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  static_cast<int>(smem_sweep)));
-    NKG_CUDA(cudaFuncSetAttribute(ppr_colsum<CPL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  static_cast<int>(smem_sweep)));
-    NKG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, ppr_sweep<CPL>, kPprThreads,
+    const size_t smem_sweep = static_cast<size_t>(kPprWarps) * 128 * sizeof(double);
+    // Wide rows: one CTA per SM, as many stages per warp as fit.
+    const bool wide = parts == 2;
+    const size_t stage_bytes = static_cast<size_t>(kBulkWarps) * kBulkArcs * kp * sizeof(float);
+    const uint32_t stages = static_cast<uint32_t>(
+        std::min<size_t>(kBulkStages, kBulkBytes / stage_bytes));
+    const size_t smem_bulk = stages * stage_bytes;
+    if (wide)
+        NKG_CUDA(cudaFuncSetAttribute(ppr_sweep_bulk, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      static_cast<int>(smem_bulk)));
+    NKG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, ppr_sweep, kPprThreads,
                                                            smem_sweep));
-    occ = std::max(occ, 1);
-    const uint32_t sweep_ctas = static_cast<uint32_t>(
-        std::max<uint64_t>(1, std::min<uint64_t>(static_cast<uint64_t>(occ) * sms,
-                                                 (nv + kPprWarps - 1) / kPprWarps)));
+    occ = wide ? 1 : std::max(occ, 1);
+    const uint32_t warps = wide ? kBulkWarps : kPprWarps;  // per CTA
+    const uint32_t sweep_ctas = static_cast<uint32_t>(std::max<uint64_t>(
+        1, std::min<uint64_t>(static_cast<uint64_t>(occ) * sms, (nv + warps - 1) / warps)));
     const uint32_t units = std::max<uint32_t>(
-        1, std::min<uint32_t>(sweep_ctas * kPprWarps * 4, std::max<uint32_t>(nv, 1)));
+        1, std::min<uint32_t>(sweep_ctas * warps * 4, std::max<uint32_t>(nv, 1)));
     DeviceArray<uint64_t> cost(std::max<uint32_t>(nv, 1)), cost_incl(std::max<uint32_t>(nv, 1));
     DeviceArray<uint32_t> unit_start(units + 1);
+    DeviceArray<uint2> vrange(std::max<uint32_t>(nv, 1));
     if (nv) {
-        ppr_vrow_cost<<<ceil_div(nv, 256), 256, 0, s>>>(g->row_ptr.get(), chunk_begin,
-                                                        chunk_row.get(), n_chunks, n_long,
-                                                        n, cost.get());
+        ppr_vrow_ranges<<<ceil_div(nv, 256), 256, 0, s>>>(g->row_ptr.get(), chunk_begin,
+                                                          chunk_row.get(), n_chunks, n_long, n,
+                                                          vrange.get(), cost.get());
         size_t tb = 0;
         NKG_CUDA(cub::DeviceScan::InclusiveSum(nullptr, tb, cost.get(), cost_incl.get(),
                                                static_cast<int64_t>(nv), s));
@@ -534,8 +775,10 @@ void run_ppr(nkg_graph *g, const nkg_pr_params &p, uint32_t k, const uint32_t *s
     }
     ppr_unit_bounds<<<ceil_div(units + 1, 256), 256, 0, s>>>(cost_incl.get(), nv, units,
                                                              unit_start.get());
+    // At most 16 rows of the sweep's partials per fix-up CTA.
     const uint32_t fix_ctas = std::max<uint32_t>(
-        1, std::min<uint32_t>(sms * 2, (n_long + kPprWarps - 1) / kPprWarps));
+        ceil_div(sweep_ctas, 16),
+        std::min<uint32_t>(sms * 2, ceil_div(static_cast<uint64_t>(n_long) * parts, kPprWarps)));
 
     // Per-call buffers.
     DeviceArray<float> y0(static_cast<size_t>(n) * kp), y1(static_cast<size_t>(n) * kp);
@@ -570,7 +813,7 @@ void run_ppr(nkg_graph *g, const nkg_pr_params &p, uint32_t k, const uint32_t *s
     a.col = g->col.get();
     a.degc = g->degc.get();
     a.chunk_begin = chunk_begin;
-    a.chunk_row = chunk_row.get();
+    a.vrange = vrange.get();
     a.unit_start = unit_start.get();
     a.seed = seed.get();
     a.chunk_val = chunk_val.get();
@@ -590,6 +833,9 @@ void run_ppr(nkg_graph *g, const nkg_pr_params &p, uint32_t k, const uint32_t *s
     a.units = units;
     a.kp = kp;
     a.sweep_ctas = sweep_ctas;
+    a.lanes = lanes;
+    a.groups = groups;
+    a.parts = parts;
     a.l2 = p.norm == NKG_NORM_L2;
     a.distribute = p.distribute_sinks ? 1 : 0;
 
@@ -599,12 +845,17 @@ void run_ppr(nkg_graph *g, const nkg_pr_params &p, uint32_t k, const uint32_t *s
         for (int i = 0; i < 8; ++i) {
             a.y_in = ((it + i) & 1) ? y1.get() : y0.get();
             a.y_out = ((it + i) & 1) ? y0.get() : y1.get();
-            ppr_sweep<CPL><<<sweep_ctas, kPprThreads, smem_sweep, s>>>(a);
-            ppr_fixup<CPL><<<fix_ctas, kPprThreads, smem_sweep, s>>>(a, fix_res.get(), fix_sink.get());
+            if (wide)
+                ppr_sweep_bulk<<<sweep_ctas, kBulkThreads, smem_bulk, s>>>(a, stages);
+            else
+                ppr_sweep<<<sweep_ctas, kPprThreads, smem_sweep, s>>>(a);
+            ppr_fixup<<<fix_ctas, kPprThreads, smem_sweep, s>>>(a, fix_res.get(), fix_sink.get());
         }
         launches += 16;
         NKG_CUDA(cudaGetLastError());
         h = read_scalar(st.get(), s);
+        if (h.error)
+            throw Error(NKG_ERR_TIMEOUT, "a row copy of the personalised PageRank sweep timed out");
         if (h.all_done)
             break;
         check_cancel(g, "personalised PageRank run cancelled");
@@ -615,8 +866,7 @@ void run_ppr(nkg_graph *g, const nkg_pr_params &p, uint32_t k, const uint32_t *s
     // Normalisation per column (PageRank.cpp:75-92), output in the caller's ids.
     const uint32_t cs_ctas = std::min<uint32_t>(sms * 2, std::max<uint32_t>((n + kPprWarps - 1) / kPprWarps, 1));
     DeviceArray<double> part_sum(static_cast<size_t>(cs_ctas) * kp), part_sink(static_cast<size_t>(cs_ctas) * kp);
-    ppr_colsum<CPL><<<cs_ctas, kPprThreads, smem_sweep, s>>>(yfin, g->degc.get(), n, kp,
-                                                             part_sum.get(), part_sink.get());
+    ppr_colsum<<<cs_ctas, kPprThreads, smem_sweep, s>>>(a, yfin, part_sum.get(), part_sink.get());
     std::vector<double> hs(static_cast<size_t>(cs_ctas) * kp), hk(static_cast<size_t>(cs_ctas) * kp);
     NKG_CUDA(cudaMemcpyAsync(hs.data(), part_sum.get(), hs.size() * sizeof(double),
                              cudaMemcpyDeviceToHost, s));
@@ -702,10 +952,6 @@ extern "C" int nkg_ppr_run(nkg_graph *g, const nkg_pr_params *p, uint32_t k, con
             require(seeds[j] < g->z, "seed id out of range");
         DeviceGuard guard(g->device);
         RunScope scope(g);
-        // CPL columns per lane (float4 loads): 128 or 256 columns per sweep.
-        if (k <= 128)
-            run_ppr<4>(g, *p, k, seeds, scores_out, out_on_device != 0, iterations_out, stats);
-        else
-            run_ppr<8>(g, *p, k, seeds, scores_out, out_on_device != 0, iterations_out, stats);
+        run_ppr(g, *p, k, seeds, scores_out, out_on_device != 0, iterations_out, stats);
     });
 }
