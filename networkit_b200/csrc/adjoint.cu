@@ -386,7 +386,7 @@ __global__ void __launch_bounds__(kAdjThreads) adj_fix(AdjArgs a) {
         td += a.part[2 * static_cast<size_t>(i) + 1];
     }
     for_split_rows<kAdjThreads, double>(
-        a.chunk_begin, a.chunk_val, a.n_long, a.n_vlong,
+        a.chunk_begin, a.chunk_val, a.n_long, a.n_vlong, 0u,
         [&](uint32_t r, double acc) { adj_row<WEIGHTED>(a, r, acc, tdot, res, td); });
     res = block_sum<kAdjThreads>(res, s_red);
     td = block_sum<kAdjThreads>(td, s_red);
@@ -940,9 +940,9 @@ AdjResult run_adjoint(nkg_graph *g, const nkg_pr_params &p, const double *d_tele
     const double inv_n = 1.0 / static_cast<double>(n);
     const unsigned vec_ctas = std::max<unsigned>(1, std::min<unsigned>(sms * 4, ceil_div(n, kBiThreads)));
     const unsigned fix_ctas = fix_ctas_with_units(
-        split_fix_ctas<kBiThreads>(A.tl.n_long, A.tl.n_vlong), A.n_units32, kBiThreads);
+        split_fix_ctas<kBiThreads>(A.tl.n_long, A.tl.n_vlong, 0), A.n_units32, kBiThreads);
     const unsigned adj_fix_ctas = fix_ctas_with_units(
-        split_fix_ctas<kAdjThreads>(A.tl.n_long, A.tl.n_vlong), A.n_units64, kAdjThreads);
+        split_fix_ctas<kAdjThreads>(A.tl.n_long, A.tl.n_vlong, 0), A.n_units64, kAdjThreads);
     ensure_work(g, A, vec_ctas, std::max(fix_ctas, adj_fix_ctas));
     AdjWork &W = A.work;
     AdjResult R;

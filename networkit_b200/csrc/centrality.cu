@@ -178,7 +178,7 @@ __global__ void __launch_bounds__(kCentFix) cent_fix(CentArgs a) {
     for (uint32_t i = blockIdx.x * kCentFix + threadIdx.x; i < a.units; i += gridDim.x * kCentFix)
         sq += a.part[i];
     for_split_rows<kCentFix, double>(
-        a.chunk_begin, a.chunk_val, a.n_long, a.n_vlong,
+        a.chunk_begin, a.chunk_val, a.n_long, a.n_vlong, a.n_hot,
         [&](uint32_t r, double acc) { cent_row<MODE>(a, r, acc, len_prev, sq); });
     sq = block_sum<kCentFix>(sq, s_red);
     if (threadIdx.x == 0) {
@@ -280,7 +280,7 @@ CentResult cent_run(nkg_graph *g, const SellLayout &L, const double *w_sell, dou
         1, std::min<uint64_t>(static_cast<uint64_t>(ctas) * (kCentThreads / 32) * kQueueUnitsPerWarp,
                               std::max<uint64_t>(slices, 1))));
     const unsigned fix_ctas =
-        fix_ctas_with_units(split_fix_ctas<kCentFix>(L.n_long, L.n_vlong), units, kCentFix);
+        fix_ctas_with_units(split_fix_ctas<kCentFix>(L.n_long, L.n_vlong, L.n_hot), units, kCentFix);
     DeviceArray<uint32_t> unit_start(static_cast<size_t>(units) + 1);
     sell_units(L, units, unit_start.get(), s);
     DeviceArray<double> x[2] = {DeviceArray<double>(n + 1), DeviceArray<double>(n + 1)};

@@ -47,10 +47,11 @@ constexpr uint32_t kMinSegment = 4;
 constexpr uint32_t kHotChunk = 128;
 // Rows of at most this many arcs have no segments.
 constexpr uint32_t kHotRow = 32;
-// Graphs below have no blocks: the launch and the copies take most of what the
-// gathers gain, and the layout takes longer to build (R-MAT 21, 32M arcs, FP64:
-// 12.4 ms a run with blocks, 12.8 without; R-MAT 22, 65M: 20.6 and 23.6).
-constexpr uint64_t kHotGraphArcs = 40ull << 20;
+// Graphs below have no blocks: building them takes 1.2 ms at 60M arcs, which
+// the first run should win back. R-MAT, runs without / with blocks: 3.8M nodes
+// (58.5M arcs, 76 iterations) 16.2 / 15.6 ms, 4.2M nodes (65.2M arcs, 103
+// iterations) 23.4 / 20.1 ms, 8.4M nodes (131M arcs) 44.7 / 32.8 ms.
+constexpr uint64_t kHotGraphArcs = 60ull << 20;
 // Rows longer than this are partitioned by a whole CTA.
 constexpr uint32_t kBigRow = 2048;
 

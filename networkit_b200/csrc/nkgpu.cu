@@ -593,7 +593,7 @@ __global__ void segment_chunks(uint32_t n_hot, uint32_t n_long, uint32_t chunk,
 // Chunks of the partitioned rows, in row order, then block order: first arc,
 // length (a segment's chunks are of equal length, give or take one arc) and
 // sort key (block, then longest first); the first chunk of every row; the
-// last row of more than kShortChunks chunks. One warp per row.
+// last row of more than kShortSums chunks. One warp per row.
 __global__ void expand_segments(const uint32_t *__restrict__ row_ptr, uint32_t n_hot,
                                 uint32_t n_long, const uint32_t *__restrict__ seg_base,
                                 const uint32_t *__restrict__ seg_cnt,
@@ -618,7 +618,7 @@ __global__ void expand_segments(const uint32_t *__restrict__ row_ptr, uint32_t n
             chunk_begin[r] = seg_chunk[sb];
             if (r == n_hot - 1)
                 chunk_begin[n_hot] = seg_chunk[sb + ns];
-            if (r < n_long && seg_chunk[sb + ns] - seg_chunk[sb] > kShortChunks)
+            if (r < n_long && seg_chunk[sb + ns] - seg_chunk[sb] > kShortSums)
                 atomicMax(vlong, r + 1);
         }
         if (!cnt)
@@ -1659,7 +1659,7 @@ static nkg_graph *build_graph(std::unique_ptr<nkg_graph> g, DeviceArray<uint64_t
     g->cta_sink.alloc(static_cast<size_t>(sms) * 32);
     // Fix-up grids also cover the queued sweep's unit partials (at most one
     // unit per slice, kUnitsPerFixThread per thread).
-    const size_t fix = fix_ctas_with_units(split_fix_ctas<kFixThreads>(g->fw.n_long, g->fw.n_vlong),
+    const size_t fix = fix_ctas_with_units(split_fix_ctas<kFixThreads>(g->fw.n_long, g->fw.n_vlong, g->fw.n_hot),
                                            g->fw.slices, kFixThreads);
     g->fix_res.alloc(fix);
     g->fix_sink.alloc(fix);
@@ -1929,7 +1929,7 @@ static void sweep_setup(nkg_graph *g) {
     unit_bounds<<<ceil_div(static_cast<uint64_t>(P.units) + 1, 256), 256, 0, s>>>(
         g->fw.slice_cost.get(), g->fw.slices, P.units, P.unit_start.get());
     NKG_CUDA(cudaGetLastError());
-    P.fix_ctas = split_fix_ctas<kFixThreads>(g->fw.n_long, g->fw.n_vlong);
+    P.fix_ctas = split_fix_ctas<kFixThreads>(g->fw.n_long, g->fw.n_vlong, g->fw.n_hot);
     P.hot = hot_tier_ids<T>(g);
     if (!P.hot) {
         // The queued sweep's units (the tier kernel keeps the static ones).
@@ -2403,7 +2403,7 @@ static RunResult run_refine(nkg_graph *g, const nkg_pr_params &p, const double *
     DeviceArray<float> &bx = W.x, &br = W.r, &brhat = W.rhat, &bp = W.p, &bv = W.v, &bs = W.s,
                        &bt = W.t, &bg = W.g;
     DeviceArray<double> &x64 = W.x64, &part = W.part;
-    const unsigned fix_ctas = fix_ctas_with_units(split_fix_ctas<kBiThreads>(g->fw.n_long, g->fw.n_vlong),
+    const unsigned fix_ctas = fix_ctas_with_units(split_fix_ctas<kBiThreads>(g->fw.n_long, g->fw.n_vlong, g->fw.n_hot),
                                                   P32.q_units, kBiThreads);
     if (W.fix_part.size() < 2 * static_cast<size_t>(fix_ctas))
         W.fix_part.alloc(2 * static_cast<size_t>(fix_ctas));

@@ -277,7 +277,7 @@ nkg_part *create_part(uint64_t vec_len, uint64_t row_base, uint64_t rows, uint64
     p->unit_start.alloc(static_cast<size_t>(p->units) + 1);
     sell_units(p->fw, p->units, p->unit_start.get(), s);
     p->fix_ctas = fix_ctas_with_units(
-        split_fix_ctas<kFixThreads>(p->fw.n_long, p->fw.n_vlong), p->units, kFixThreads);
+        split_fix_ctas<kFixThreads>(p->fw.n_long, p->fw.n_vlong, 0), p->units, kFixThreads);
     p->chunk_val.alloc(static_cast<size_t>(p->fw.s_chunk) * 32 + 1);
     p->unit_part.alloc(2 * static_cast<size_t>(p->units));
     p->fix_res.alloc(p->fix_ctas);

@@ -247,7 +247,7 @@ __global__ void __launch_bounds__(kBiThreads) bi_mv_fix(BiArgs a) {
         }
     }
     for_split_rows<kBiThreads, float>(
-        a.chunk_begin, a.chunk_val, a.n_long, a.n_vlong, [&](uint32_t r, float acc) {
+        a.chunk_begin, a.chunk_val, a.n_long, a.n_vlong, a.n_hot, [&](uint32_t r, float acc) {
             bi_mv_row<WEIGHTED, MODE, OP>(a, r, acc, px, out, d1, d2);
         });
     d1 = block_sum<kBiThreads>(d1, s_red);

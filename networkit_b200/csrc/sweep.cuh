@@ -45,9 +45,13 @@ inline uint32_t chunk_for(uint64_t arcs, unsigned sms) {
     return arcs >= static_cast<uint64_t>(sms) * 48 * 32 * 160 ? kChunk : kSmallChunk;
 }
 // A split row with more chunk sums than this is summed by a whole warp in the
-// fix-up, the others by kRowLanes lanes.
-constexpr uint32_t kShortChunks = 128;
-constexpr uint32_t kRowLanes = 8;
+// fix-up, the others by one thread. With source blocks (hot.cuh) a row has a
+// dozen sums and eight lanes; without, two or three: eight lanes a row took 19
+// us of an iteration on 58M arcs, a thread a row 12.5 (iteration 0.223 / 0.209
+// ms).
+constexpr uint32_t kShortChunks = 16;
+constexpr uint32_t kShortSums = 128;
+__host__ __device__ inline uint32_t row_lanes(uint32_t n_hot) { return n_hot ? 8u : 1u; }
 
 // Work units of the queued sweeps: warp gw of nw runs unit gw first, with no
 // ticket, then units nw + t for the tickets t it takes from `queue`, while
@@ -124,7 +128,7 @@ struct SweepArgs {
     IterState *st;
     uint32_t n;
     uint32_t n_long;        // rows [0, n_long) are split into chunks
-    uint32_t n_vlong;       // rows [0, n_vlong) have more than kShortChunks chunks
+    uint32_t n_vlong;       // rows [0, n_vlong) are summed by a warp each
     uint32_t s_chunk;       // slices [0, s_chunk) hold chunks, the rest rows
     uint32_t units;
     uint32_t sweep_ctas;
@@ -492,11 +496,12 @@ __global__ void __launch_bounds__(THREADS, UNROLL != 8 || (WEIGHTED && sizeof(T)
 constexpr int kFixThreads = 256;
 
 // CTAs of THREADS threads that finish the split rows (for_split_rows): a warp
-// for each row of more than kShortChunks chunk sums, then kRowLanes lanes for
-// each other row, at most 8 CTAs per SM of them.
+// for each of the first n_vlong rows, then row_lanes() lanes for each other
+// row, at most 8 CTAs per SM of them.
 template <int THREADS>
-inline unsigned split_fix_ctas(uint32_t n_long, uint32_t n_vlong) {
-    constexpr uint32_t w = THREADS / 32, rows = THREADS / kRowLanes;
+inline unsigned split_fix_ctas(uint32_t n_long, uint32_t n_vlong, uint32_t n_hot) {
+    constexpr uint32_t w = THREADS / 32;
+    const uint32_t rows = THREADS / row_lanes(n_hot);
     const uint64_t short_rows = n_long > n_vlong ? n_long - n_vlong : 0;
     return static_cast<unsigned>(std::max<uint64_t>(
         1, (n_vlong + w - 1) / w + std::min<uint64_t>(1184, (short_rows + rows - 1) / rows)));
@@ -527,15 +532,16 @@ __device__ __forceinline__ V lane_chunk_sum(const V *__restrict__ v, uint32_t cb
 
 // Calls finish(r, sum) once for every split row r < n_long with the sum of its
 // chunk sums, in a fixed order: a warp for each of the first n_vlong rows
-// (lane-strided partials in V, then across lanes in double), kRowLanes lanes
+// (lane-strided partials in V, then across lanes in double), row_lanes() lanes
 // for each other (four loads of a lane in flight; one thread per row took 42
 // us of every R-MAT 24 iteration where source blocks give a row a dozen sums).
 // Every thread of the CTA calls it.
 template <int THREADS, typename V, typename F>
 __device__ __forceinline__ void for_split_rows(const uint32_t *__restrict__ chunk_begin,
                                                const V *__restrict__ chunk_val, uint32_t n_long,
-                                               uint32_t n_vlong, F &&finish) {
-    constexpr uint32_t w = THREADS / 32, rows = THREADS / kRowLanes;
+                                               uint32_t n_vlong, uint32_t n_hot, F &&finish) {
+    constexpr uint32_t w = THREADS / 32;
+    const uint32_t lanes = row_lanes(n_hot), shift = n_hot ? 3 : 0, rows = THREADS >> shift;
     const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const uint32_t vctas = (n_vlong + w - 1) / w;
     if (blockIdx.x < vctas) {
@@ -549,25 +555,24 @@ __device__ __forceinline__ void for_split_rows(const uint32_t *__restrict__ chun
             finish(r, acc);
         return;
     }
-    const uint32_t sub = lane % kRowLanes;
+    const uint32_t sub = lane & (lanes - 1);
     const uint32_t stride = (gridDim.x - vctas) * rows;
-    for (uint32_t base = n_vlong + (blockIdx.x - vctas) * rows + wid * (32 / kRowLanes);
+    for (uint32_t base = n_vlong + (blockIdx.x - vctas) * rows + wid * (32u >> shift);
          base < n_long; base += stride) {
-        const uint32_t r = base + lane / kRowLanes;
+        const uint32_t r = base + (lane >> shift);
         const uint32_t e = r < n_long ? chunk_begin[r + 1] : 0u;
         V sum = V(0);
-        for (uint32_t k = r < n_long ? chunk_begin[r] + sub : 0u; k < e; k += 4 * kRowLanes) {
+        for (uint32_t k = r < n_long ? chunk_begin[r] + sub : 0u; k < e; k += 4 * lanes) {
             V x[4];
 #pragma unroll
             for (uint32_t q = 0; q < 4; ++q)
-                x[q] = k + q * kRowLanes < e ? chunk_val[k + q * kRowLanes] : V(0);
+                x[q] = k + q * lanes < e ? chunk_val[k + q * lanes] : V(0);
 #pragma unroll
             for (uint32_t q = 0; q < 4; ++q)
                 sum += x[q];
         }
         __syncwarp();
-#pragma unroll
-        for (uint32_t o = kRowLanes / 2; o > 0; o >>= 1)
+        for (uint32_t o = lanes / 2; o > 0; o >>= 1)
             sum += __shfl_xor_sync(0xffffffffu, sum, o);
         if (sub == 0 && r < n_long)
             finish(r, sum);
@@ -592,7 +597,7 @@ __global__ void __launch_bounds__(kFixThreads) fixup_kernel(SweepArgs<T> a) {
         }
     }
     for_split_rows<kFixThreads, T>(
-        a.chunk_begin, a.chunk_val, a.n_long, a.n_vlong, [&](uint32_t r, T sum) {
+        a.chunk_begin, a.chunk_val, a.n_long, a.n_vlong, a.n_hot, [&](uint32_t r, T sum) {
             finish_row<T, WEIGHTED, PART>(a, rp, sink_coef, r, sum, res, sink);
         });
     const double bres = block_sum<kFixThreads>(res, s_red);

@@ -18,9 +18,9 @@ THREADS = os.cpu_count() or 1
 def rmat():
     """R-MAT 22: large enough for source blocks, hubs of tens of thousands of
     arcs (partitioned by a whole CTA)."""
-    csr = generators.rmat_directed(22, 12, seed=7)
+    csr = generators.rmat_directed(22, 18, seed=7)
     dg = _capi.DeviceGraph(csr)
-    assert csr.arcs >= 40 << 20  # smaller graphs have none
+    assert csr.arcs >= 60 << 20  # smaller graphs have none
     return csr, dg
 
 
