@@ -1436,8 +1436,12 @@ def main():
                        "wall_s": wall, "ms_create": info["ms_create"]},
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": profiled_traffic(
-                             f"sweep_fp64_rmat{args.scale}"),
-                         "kernel": "sweep_kernel<double> (SELL-32 pull SpMV)",
+                             f"sweep_source_blocks_rmat{args.scale}"
+                             if args.hot_tier_kb < 0 else f"sweep_fp64_rmat{args.scale}"),
+                         "kernel": "hot_kernel<double> + sweep_kernel<double> "
+                                   "(SELL-32 pull SpMV with source blocks)"
+                                   if args.hot_tier_kb < 0 else
+                                   "sweep_kernel<double> (SELL-32 pull SpMV)",
                          "bytes_per_launch": bytes_sweep, "ms_per_launch": ms_kernel,
                          "ms_per_iteration": ms_iter, "peak_source": peak_kind,
                          "gather_bound_ms": ms_gather,
