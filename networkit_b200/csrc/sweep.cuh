@@ -46,12 +46,13 @@ inline uint32_t chunk_for(uint64_t arcs, unsigned sms) {
 }
 // A split row with more chunk sums than this is summed by a whole warp in the
 // fix-up, the others by one thread. With source blocks (hot.cuh) a row has a
-// dozen sums and eight lanes; without, two or three: eight lanes a row took 19
-// us of an iteration on 58M arcs, a thread a row 12.5 (iteration 0.223 / 0.209
-// ms).
+// dozen sums and four lanes (R-MAT 24, FP64 iteration with four / eight
+// lanes: 0.636 / 0.641 ms); without, two or three: eight lanes a row took
+// 19 us of an iteration on 58M arcs, a thread a row 12.5 (iteration 0.223 /
+// 0.209 ms).
 constexpr uint32_t kShortChunks = 16;
 constexpr uint32_t kShortSums = 128;
-__host__ __device__ inline uint32_t row_lanes(uint32_t n_hot) { return n_hot ? 8u : 1u; }
+__host__ __device__ inline uint32_t row_lanes(uint32_t n_hot) { return n_hot ? 4u : 1u; }
 
 // Work units of the queued sweeps: warp gw of nw runs unit gw first, with no
 // ticket, then units nw + t for the tickets t it takes from `queue`, while
@@ -497,14 +498,15 @@ constexpr int kFixThreads = 256;
 
 // CTAs of THREADS threads that finish the split rows (for_split_rows): a warp
 // for each of the first n_vlong rows, then row_lanes() lanes for each other
-// row, at most 8 CTAs per SM of them.
+// row. With source blocks no more CTAs than are resident at once (4 per SM; R-MAT
+// 24, eight lanes: 0.641 ms an iteration, 0.645 with 8 per SM, 0.654 with 2).
 template <int THREADS>
 inline unsigned split_fix_ctas(uint32_t n_long, uint32_t n_vlong, uint32_t n_hot) {
     constexpr uint32_t w = THREADS / 32;
     const uint32_t rows = THREADS / row_lanes(n_hot);
     const uint64_t short_rows = n_long > n_vlong ? n_long - n_vlong : 0;
     return static_cast<unsigned>(std::max<uint64_t>(
-        1, (n_vlong + w - 1) / w + std::min<uint64_t>(1184, (short_rows + rows - 1) / rows)));
+        1, (n_vlong + w - 1) / w + std::min<uint64_t>(n_hot ? 592 : 1184, (short_rows + rows - 1) / rows)));
 }
 
 // Lane-strided partial sum of one split row's chunk partials
@@ -541,7 +543,7 @@ __device__ __forceinline__ void for_split_rows(const uint32_t *__restrict__ chun
                                                const V *__restrict__ chunk_val, uint32_t n_long,
                                                uint32_t n_vlong, uint32_t n_hot, F &&finish) {
     constexpr uint32_t w = THREADS / 32;
-    const uint32_t lanes = row_lanes(n_hot), shift = n_hot ? 3 : 0, rows = THREADS >> shift;
+    const uint32_t lanes = row_lanes(n_hot), shift = n_hot ? 2 : 0, rows = THREADS >> shift;
     const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const uint32_t vctas = (n_vlong + w - 1) / w;
     if (blockIdx.x < vctas) {
