@@ -687,9 +687,11 @@ void batch_split(nkg_batch *b) {
         NKG_CUDA(cudaMemcpyAsync(S.smem.get(), small.data(), small.size() * 4,
                                  cudaMemcpyHostToDevice, s));
         auto kfn = batch_smem_kernel<T>;
-        S.smem_bytes = (static_cast<size_t>(max_n) + 8) * sizeof(T) / 16 * 16 + 16;
-        NKG_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      static_cast<int>(S.smem_bytes)));
+        S.smem_bytes = smem_launch_bytes<T>(max_n);
+        // The attribute is the process's, so every batch sets it to the same most.
+        NKG_CUDA(cudaFuncSetAttribute(
+            kfn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+            static_cast<int>(smem_launch_bytes<T>(smem_max_nodes<T>()))));
         double best = 1e300;
         for (unsigned c = 1; c <= kSmemMaxCluster; c *= 2) {
             cudaLaunchAttribute attr;

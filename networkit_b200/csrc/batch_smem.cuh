@@ -29,6 +29,11 @@ template <typename T>
 constexpr uint32_t smem_max_nodes() {
     return static_cast<uint32_t>(kSmemBytes / sizeof(T)) - 8;
 }
+// Shared memory of a launch whose largest graph has max_n nodes.
+template <typename T>
+constexpr size_t smem_launch_bytes(uint32_t max_n) {
+    return (static_cast<size_t>(max_n) + 8) * sizeof(T) / 16 * 16 + 16;
+}
 constexpr int kSmemMaxCluster = 8;
 
 struct SmemMeta {

@@ -1959,7 +1959,9 @@ static void sweep_setup(nkg_graph *g) {
         // Carve out only what the CTAs need, leaving the rest of the SM's L1
         // to the gathers.
         const int carve = std::min(100, (copies * per_cta) * 100 / sm_smem + 1);
-        NKG_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+        // The process's most, whatever this graph's tier: others launch the kernel too.
+        NKG_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      static_cast<int>(kHotMaxBytes)));
         NKG_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributePreferredSharedMemoryCarveout, carve));
         int hocc = 0;
         NKG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&hocc, kfn, P.hot_threads, bytes));

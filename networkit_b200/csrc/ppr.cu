@@ -748,9 +748,9 @@ void run_ppr(nkg_graph *g, const nkg_pr_params &p, uint32_t k, const uint32_t *s
     const uint32_t stages = static_cast<uint32_t>(
         std::min<size_t>(kBulkStages, kBulkBytes / stage_bytes));
     const size_t smem_bulk = stages * stage_bytes;
-    if (wide)
+    if (wide)  // the kernel's own most, not this call's: other handles launch it too
         NKG_CUDA(cudaFuncSetAttribute(ppr_sweep_bulk, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      static_cast<int>(smem_bulk)));
+                                      static_cast<int>(kBulkBytes)));
     NKG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, ppr_sweep, kPprThreads,
                                                            smem_sweep));
     occ = wide ? 1 : std::max(occ, 1);
