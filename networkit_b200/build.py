@@ -30,7 +30,8 @@ GEN_LIB = os.path.join(LIBDIR, "libnkgen.so")
 
 GPU_SOURCES = ["nkgpu.cu", "noalloc.cu", "ppr.cu", "adjoint.cu", "batch.cu", "centrality.cu",
                "local.cu", "part.cu", "nkbg.cu"]
-GPU_HEADERS = ["common.cuh", "sweep.cuh", "hot.cuh", "small.cuh", "batch_smem.cuh", "refine.cuh", "graph.hpp", "host.hpp"]
+GPU_HEADERS = ["common.cuh", "sweep.cuh", "hot.cuh", "small.cuh", "batch_smem.cuh", "refine.cuh", "graph.hpp", "host.hpp",
+               "testing.h"]
 GEN_SOURCES = ["graphgen.cpp", "graphio.cpp"]
 # Restatements of the reference's generators: compiled as the reference is
 # (baseline x86-64, no floating-point contraction) so that they round alike.

@@ -766,7 +766,7 @@ namespace {
 
 // Slot -> caller arc maps of both layouts (first weight update only).
 void ensure_weight_maps(nkg_graph *g, AdjointState &A) {
-    if (A.fw_map)
+    if (A.tchunk)  // allocated last
         return;
     cudaStream_t s = g->stream;
     const uint32_t n = static_cast<uint32_t>(g->n);

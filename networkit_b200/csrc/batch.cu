@@ -524,6 +524,7 @@ struct nkg_batch {
     DeviceArray<SmemItem> sitem;
     DeviceArray<uint4> sarcs;
     uint64_t s_entries = 0;                    // entries of their iterates
+    bool smem_ready = false;
     DeviceArray<float> sy32[2];
     DeviceArray<double> sy64[2];
     BatchSplit splits[2];                      // [FP32, FP64]
@@ -545,6 +546,7 @@ void batch_layout(nkg_batch *b, uint32_t split) {
         return;
     cudaStream_t s = b->stream;
     const uint32_t count = b->count;
+    b->col_sell.reset();  // no layout until the new one is complete
     bt_split<<<ceil_div(count, 128), 128, 0, s>>>(b->meta.get(), count, b->rowlen.get(), split);
     NKG_CUDA(cudaGetLastError());
     NKG_CUDA(cudaMemcpyAsync(b->meta_h.data(), b->meta.get(), count * sizeof(GraphMeta),
@@ -589,7 +591,7 @@ void batch_layout(nkg_batch *b, uint32_t split) {
 
 // Items and arcs of the graphs that fit into shared memory in FP32.
 void smem_layout(nkg_batch *b) {
-    if (b->smeta)
+    if (b->smem_ready)
         return;
     cudaStream_t s = b->stream;
     const uint32_t count = b->count;
@@ -635,6 +637,7 @@ void smem_layout(nkg_batch *b) {
         NKG_CUDA(cudaGetLastError());
     }
     NKG_CUDA(cudaStreamSynchronize(s));
+    b->smem_ready = true;
 }
 
 cudaLaunchConfig_t smem_config(unsigned cluster, unsigned grid, size_t bytes, cudaStream_t s,

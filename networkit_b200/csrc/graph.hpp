@@ -161,6 +161,7 @@ struct Plane {
     DeviceArray<uint32_t> q_unit_start;
     DeviceArray<double> q_part;
     uint32_t q_units = 0;
+    bool ready = false;          // sweep_setup is done
     HotRun<T> hot_run;           // source blocks (hot.cuh), before every sweep
     // The sweep's last CTA closes each iteration (no fix-up launch): graphs
     // with no split rows and at most kCloseInSweepUnits units.

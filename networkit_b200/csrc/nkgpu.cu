@@ -21,6 +21,7 @@
 
 #include "graph.hpp"
 #include "host.hpp"
+#include "testing.h"
 #include "refine.cuh"
 
 using namespace nkg;
@@ -57,7 +58,13 @@ void release_blocks(BlockCache &c) {
 
 }  // namespace
 
+// Device allocations of this thread until one reports that memory ran out
+// (nkg_test_fail_alloc); negative: none does.
+static thread_local int64_t t_allocs_until_failure = -1;
+
 void *device_alloc(size_t bytes, int &device) {
+    if (t_allocs_until_failure >= 0 && t_allocs_until_failure-- == 0)
+        throw Error(NKG_ERR_OOM, "device allocation refused by nkg_test_fail_alloc");
     NKG_CUDA(cudaGetDevice(&device));
     require(device >= 0 && device < kMaxDevices, "device ordinal out of range");
     {
@@ -1890,7 +1897,7 @@ static uint32_t hot_tier_ids(const nkg_graph *g) {
 template <typename T, bool WEIGHTED>
 static void sweep_setup(nkg_graph *g) {
     Plane<T> &P = plane<T>(g);
-    if (P.y[0])
+    if (P.ready)
         return;
     cudaStream_t s = g->stream;
     const uint64_t n = g->n;
@@ -1982,6 +1989,7 @@ static void sweep_setup(nkg_graph *g) {
     require(P.sweep_ctas <= g->cta_res.size() && P.fix_ctas <= g->fix_res.size(),
             "partial-sum buffers too small");
     NKG_CUDA(cudaStreamSynchronize(s));
+    P.ready = true;
 }
 
 template <typename T, bool WEIGHTED>
@@ -2391,7 +2399,7 @@ static RunResult run_refine(nkg_graph *g, const nkg_pr_params &p, const double *
     }
     const unsigned vec_ctas = std::max<unsigned>(1, std::min<unsigned>(sms * 4, ceil_div(n, kBiThreads)));
     RefineWork &W = g->refine_work;
-    if (!W.x64) {
+    if (!W.sc) {  // allocated last
         for (auto *v : {&W.x, &W.r, &W.rhat, &W.p, &W.v, &W.s, &W.t})
             v->alloc(n);
         W.g.alloc(n + 1, 4);
@@ -2751,6 +2759,12 @@ extern "C" {
 const char *nkg_last_error(void) { return nkg::g_last_error.c_str(); }
 
 int nkg_abi_version(void) { return NKG_ABI_VERSION; }
+
+int64_t nkg_test_fail_alloc(int64_t after) {
+    const int64_t left = nkg::t_allocs_until_failure;
+    nkg::t_allocs_until_failure = after;
+    return left;
+}
 
 int nkg_release_cached_memory(int device) {
     return guarded([&] {

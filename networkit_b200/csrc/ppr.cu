@@ -727,12 +727,13 @@ void run_ppr(nkg_graph *g, const nkg_pr_params &p, uint32_t k, const uint32_t *s
 
     // Virtual rows and their cost-balanced units.
     if (!g->rc_begin) {
-        DeviceArray<uint32_t> rowlen(n);
+        DeviceArray<uint32_t> rowlen(n), begin;
         ppr_row_lengths<<<ceil_div(n, 256), 256, 0, s>>>(g->row_ptr.get(), n, rowlen.get());
         NKG_CUDA(cudaGetLastError());
         uint32_t vlong = 0;
-        g->rc_chunks = row_chunks(rowlen.get(), n, kChunk, g->rc_long, vlong, g->rc_begin, s);
+        g->rc_chunks = row_chunks(rowlen.get(), n, kChunk, g->rc_long, vlong, begin, s);
         NKG_CUDA(cudaStreamSynchronize(s));
+        g->rc_begin = std::move(begin);  // complete, or not there
     }
     const uint32_t n_long = g->rc_long, n_chunks = g->rc_chunks;
     const uint32_t *chunk_begin = g->rc_begin.get();

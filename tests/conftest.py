@@ -34,3 +34,17 @@ def load_golden(name):
 def oracle_mod():
     import oracle
     return oracle
+
+
+@pytest.fixture
+def fail_alloc():
+    """fail_alloc(k): the library's device allocation number k from now on this
+    thread fails as if memory had run out (csrc/testing.h); negative: none.
+    Returns how many were still to come before the failure set earlier."""
+    import ctypes as C
+
+    from networkit_b200 import _capi
+    f = _capi.lib().nkg_test_fail_alloc
+    f.restype, f.argtypes = C.c_int64, [C.c_int64]
+    yield f
+    f(-1)
