@@ -9,11 +9,11 @@
 // 40 columns, where rows padded to 128 columns moved 3.2 times the bytes).
 // A virtual row is a whole row, or a kChunk-arc chunk of a long row; warps
 // walk contiguous, cost-balanced ranges of them, so every sum has a fixed
-// order. Up to 128 columns (ppr_sweep) a lane holds 4 columns of a row and the
+// order. Up to 64 columns (ppr_sweep) a lane holds 4 columns of a row and the
 // warp's groups of `lanes` lanes take different arcs of the same row (37
-// columns: 3 arcs at a time); the groups' sums are added at the row's end. Rows of more than 128 columns
-// (ppr_sweep_bulk) come as bulk copies through shared memory. The other kernels treat a row of
-// more than 128 columns as two parts, each the work of its own warp.
+// columns: 3 arcs at a time); the groups' sums are added at the row's end. With
+// more columns (ppr_sweep_one) the whole warp takes one arc. The other kernels
+// treat a row of more than 128 columns as two parts, each the work of its own warp.
 #include <cub/cub.cuh>
 
 #include <algorithm>
@@ -35,8 +35,6 @@ struct PprState {
     unsigned long long iteration;
     int all_done;
     unsigned int ticket;
-    int error;  // a bulk copy did not arrive
-    int pad;
 };
 
 struct PprArgs {
@@ -148,20 +146,21 @@ __device__ __forceinline__ float finish_column(const PprArgs &a, uint32_t r, uin
     return x;
 }
 
-// Finish row r for this lane's columns. What is constant per column is loaded
+// Finish row r in columns col .. + 3. What is constant per column is loaded
 // here: held across the gathers it made the sweep spill at 64 registers.
-__device__ __forceinline__ void finish(const PprArgs &a, const PprLane &L, uint32_t r,
-                                       const float (&acc)[4], double (&res)[4], double (&sink)[4]) {
-    const int4 on = __ldg(reinterpret_cast<const int4 *>(a.active + L.col));
-    const uint4 sd = __ldg(reinterpret_cast<const uint4 *>(a.seed + L.col));
-    const float4 s4 = a.distribute ? __ldg(reinterpret_cast<const float4 *>(a.sink_coef + L.col))
+template <typename Sink>
+__device__ __forceinline__ void finish(const PprArgs &a, uint32_t col, uint32_t r,
+                                       const float (&acc)[4], double (&res)[4], Sink &&sink) {
+    const int4 on = __ldg(reinterpret_cast<const int4 *>(a.active + col));
+    const uint4 sd = __ldg(reinterpret_cast<const uint4 *>(a.seed + col));
+    const float4 s4 = a.distribute ? __ldg(reinterpret_cast<const float4 *>(a.sink_coef + col))
                                    : make_float4(0.f, 0.f, 0.f, 0.f);
     const int act[4] = {on.x, on.y, on.z, on.w};
     const uint32_t seed[4] = {sd.x, sd.y, sd.z, sd.w};
     const float sc[4] = {s4.x, s4.y, s4.z, s4.w};
     const uint32_t dc = ld_stream(a.degc + r);
     const float deg = static_cast<float>(dc);
-    const size_t at = static_cast<size_t>(r) * a.kp + L.col;
+    const size_t at = static_cast<size_t>(r) * a.kp + col;
     const float dampf = static_cast<float>(a.damp), omd = static_cast<float>(1.0 - a.damp);
     const float4 yo4 = __ldg(reinterpret_cast<const float4 *>(a.y_in + at));
     const float yo[4] = {yo4.x, yo4.y, yo4.z, yo4.w};
@@ -207,238 +206,110 @@ __device__ __forceinline__ void column_partials(const PprArgs &a, const PprLane 
     __threadfence();  // partials visible device-wide before any ticket
 }
 
-// ---------------------------------------------------------------------------
-// The sweep of wide rows (more than 128 columns): the rows of a unit's arcs
-// are bulk copies into a ring of shared memory per warp, issued along the
-// arcs of the unit without regard to row bounds, so that about 190 KB per SM
-// are in flight all the time. With the rows loaded into registers (4 arcs of
-// 1 KB per warp, 16 warps per SM) every row's end left the warp with nothing
-// in flight for two dependent loads.
-constexpr int kBulkWarps = 16;
-constexpr int kBulkThreads = kBulkWarps * 32;
-constexpr uint32_t kBulkArcs = 4;        // arcs per stage
-constexpr uint32_t kBulkStages = 8;      // most stages of a warp's ring
-constexpr uint32_t kBulkPolls = 1u << 20;  // a wait gives up after about a second
-constexpr size_t kBulkBytes = 216 * 1024;
-
-__device__ __forceinline__ uint32_t smem_addr(const void *p) {
-    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-__device__ __forceinline__ void bar_init(uint64_t *b) {
-    asm volatile("mbarrier.init.shared.b64 [%0], 1;" ::"r"(smem_addr(b)) : "memory");
-}
-__device__ __forceinline__ void bar_expect(uint64_t *b, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared.b64 _, [%0], %1;" ::"r"(smem_addr(b)), "r"(bytes)
-                 : "memory");
-}
-// True once the phase is complete; false when the wait ran out.
-__device__ __forceinline__ bool bar_wait(uint64_t *b, uint32_t phase) {
-    for (uint32_t i = 0; i < kBulkPolls; ++i) {
-        uint32_t ok;
-        asm volatile("{\n .reg .pred p;\n"
-                     " mbarrier.try_wait.parity.shared.b64 p, [%1], %2;\n"
-                     " selp.u32 %0, 1, 0, p;\n}"
-                     : "=r"(ok)
-                     : "r"(smem_addr(b)), "r"(phase)
-                     : "memory");
-        if (ok)
-            return true;
-    }
-    return false;
-}
-__device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t bytes, uint64_t *b) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                 ::"r"(smem_addr(dst)), "l"(src), "r"(bytes), "r"(smem_addr(b))
-                 : "memory");
-}
-
-// One warp's ring over the arcs [next, end): stages of kBulkArcs rows.
-struct PprRing {
-    unsigned char *rows;  // the warp's stages
-    uint64_t *bar;
-    uint32_t stages, row_bytes;
-    uint32_t begin, next, end;  // next arc to issue
-    uint32_t window;            // sources of the 32 arcs the next one lies in
-    uint32_t fill, phases;      // stage to fill; parity of every stage's next wait
-};
-
-__device__ __forceinline__ void ring_issue(const PprArgs &a, PprRing &q) {
-    const uint32_t lane = threadIdx.x & 31;
-    const uint32_t n = min(kBulkArcs, q.end - q.next);
-    if (!n)
-        return;
-    const uint32_t at = (q.next - q.begin) & 31;
-    if (at == 0)
-        q.window = q.next + lane < q.end ? ld_stream(a.col + q.next + lane) : 0u;
-    const uint32_t src = __shfl_sync(0xffffffffu, q.window, (at + lane) & 31);
-    if (lane == 0)
-        bar_expect(q.bar + q.fill, n * q.row_bytes);
-    __syncwarp();
-    if (lane < n)
-        bulk_load(q.rows + (q.fill * kBulkArcs + lane) * q.row_bytes,
-                  a.y_in + static_cast<size_t>(src) * a.kp, q.row_bytes, q.bar + q.fill);
-    q.next += n;
-    q.fill = q.fill + 1 == q.stages ? 0 : q.fill + 1;
-}
-
-// A lane holds columns h * 128 + 4 lane ..+3 for h = 0, 1.
-__global__ void __launch_bounds__(kBulkThreads, 1) ppr_sweep_bulk(PprArgs a, uint32_t stages) {
-    constexpr int H = 2;
-    extern __shared__ __align__(128) unsigned char s_ring[];
-    __shared__ uint64_t s_bar[kBulkWarps][kBulkStages];
+// The sweep of more than 64 columns: all lanes of a warp take the same arc, a
+// lane holding 4 H columns of it (H 2: more than 128 columns). Its gathers are
+// unconditional (lanes past the columns load the first ones, arcs past a row's
+// last whole batch go one by one): with loads under a condition, as ppr_sweep
+// has them, the compiler branches around each and the four of a batch no longer
+// overlap. Bound by L2 and DRAM on random rows and by the row ends, where a warp
+// has nothing in flight: 24 warps per SM for H 2 (80 registers; the sink sums,
+// which few rows add to, are in shared memory), 32 for H 1. 16 sweeps, ms, with
+// the rows as bulk copies into shared memory instead / now: 256 columns R-MAT 20
+// 59.8 / 41.6, hyperbolic 1M 48.2 / 39.6, Barabasi-Albert 4M 204 / 205,
+// Erdos-Renyi 1M 37.5 / 37.9; 129 columns 52.8 / 33.5, 44.6 / 33.5, 178 / 168,
+// 32.7 / 32.5. The copies go past L1 and cost an issue slot each, so they lost
+// where sources repeat and won nowhere by more than 1%. H 1 against ppr_sweep:
+// R-MAT 22, 128 columns 75.1 / 89.2, 68 columns 66.6 / 83.7.
+template <int H>
+__global__ void __launch_bounds__(kPprThreads, H == 1 ? 4 : 3) ppr_sweep_one(PprArgs a) {
+    extern __shared__ double s_buf[];
     if (*(volatile int *)&a.st->all_done)
         return;
     const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    if (lane == 0)
-        for (uint32_t i = 0; i < stages; ++i)
-            bar_init(&s_bar[wid][i]);
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    asm volatile("fence.proxy.async;" ::: "memory");
-    __syncwarp();
-    const float dampf = static_cast<float>(a.damp), omd = static_cast<float>(1.0 - a.damp);
-    bool on[H];
-    int act[H][4];
-    float sc[H][4];
-    uint32_t seed[H][4];
-    double res[H][4], sink[H][4];
+    const bool on = lane * 4 * H < a.kp;
+    const uint32_t col = on ? lane * 4 * H : 0;
+    double res[H][4];
+    double *sink = s_buf + wid * a.kp + col;
 #pragma unroll
-    for (int h = 0; h < H; ++h) {
-        const uint32_t c0 = h * 128 + lane * 4;
-        on[h] = c0 < a.kp;
+    for (int h = 0; h < H; ++h)
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-            act[h][c] = on[h] ? a.active[c0 + c] : 0;
-            sc[h][c] = on[h] ? a.sink_coef[c0 + c] : 0.f;
-            seed[h][c] = on[h] ? a.seed[c0 + c] : kNone;
-            res[h][c] = sink[h][c] = 0.0;
+            res[h][c] = 0.0;
+            if (on)
+                sink[4 * h + c] = 0.0;
         }
-    }
-    PprRing q;
-    q.row_bytes = a.kp * 4;
-    q.stages = stages;
-    q.rows = s_ring + static_cast<size_t>(wid) * stages * kBulkArcs * q.row_bytes;
-    q.bar = s_bar[wid];
-    q.fill = 0;
-    q.phases = 0;
-    q.window = 0;
-    uint32_t cur = 0;  // stage to read next
-    bool ok = true;
-    const uint32_t gw = blockIdx.x * kBulkWarps + wid, nw = gridDim.x * kBulkWarps;
-    for (uint32_t u = gw; u < a.units && ok; u += nw) {
+    const float *ycol = a.y_in + col;
+    const uint32_t gw = blockIdx.x * kPprWarps + wid, nw = gridDim.x * kPprWarps;
+    for (uint32_t u = gw; u < a.units; u += nw) {
         const uint32_t v_end = a.unit_start[u + 1];
-        uint32_t v = a.unit_start[u];
-        if (v >= v_end)
-            continue;
-        q.begin = q.next = __ldg(a.vrange + v).x;
-        q.end = __ldg(a.vrange + v_end - 1).y;
-        for (uint32_t i = 0; i < stages; ++i)
-            ring_issue(a, q);
-        uint32_t k = q.begin;
-        uint32_t e = __ldg(a.vrange + v).y;
-        float acc[H][4];
-        float4 yo[H];
-        uint32_t dc = 0;
-        // Row v's own entries, wanted at its end, are loaded at its start.
-        auto open_row = [&]() {
+        for (uint32_t v = a.unit_start[u]; v < v_end; ++v) {
+            const uint2 arcs = __ldg(a.vrange + v);
+            float acc[H][4];
 #pragma unroll
-            for (int h = 0; h < H; ++h) {
+            for (int h = 0; h < H; ++h)
 #pragma unroll
                 for (int c = 0; c < 4; ++c)
                     acc[h][c] = 0.f;
-                yo[h] = make_float4(0.f, 0.f, 0.f, 0.f);
-            }
-            if (v >= a.n_chunks) {
-                const uint32_t r = a.n_long + (v - a.n_chunks);
-                dc = ld_stream(a.degc + r);
+            for (uint32_t base = arcs.x; base < arcs.y; base += 32) {
+                const uint32_t cnt = min(32u, arcs.y - base);
+                const uint32_t cl = lane < cnt ? ld_stream(a.col + base + lane) : 0u;
+                uint32_t i = 0;
+                for (; i + kPprBatch <= cnt; i += kPprBatch) {
+                    float4 x[kPprBatch][H];
 #pragma unroll
-                for (int h = 0; h < H; ++h)
-                    if (on[h])
-                        yo[h] = __ldg(reinterpret_cast<const float4 *>(
-                            a.y_in + static_cast<size_t>(r) * a.kp + h * 128 + lane * 4));
-            }
-        };
-        auto close_row = [&]() {
-            if (v < a.n_chunks) {
+                    for (uint32_t q = 0; q < kPprBatch; ++q) {
+                        const uint32_t src = __shfl_sync(0xffffffffu, cl, i + q);
+                        const float4 *y =
+                            reinterpret_cast<const float4 *>(ycol + static_cast<size_t>(src) * a.kp);
 #pragma unroll
-                for (int h = 0; h < H; ++h)
-                    if (on[h])
-                        *reinterpret_cast<float4 *>(a.chunk_val + static_cast<size_t>(v) * a.kp +
-                                                    h * 128 + lane * 4) =
-                            make_float4(acc[h][0], acc[h][1], acc[h][2], acc[h][3]);
-                return;
+                        for (int h = 0; h < H; ++h)
+                            x[q][h] = __ldg(y + h);
+                    }
+#pragma unroll
+                    for (uint32_t q = 0; q < kPprBatch; ++q)
+#pragma unroll
+                        for (int h = 0; h < H; ++h)
+                            add4(acc[h], x[q][h]);
+                }
+                for (; i < cnt; ++i) {
+                    const uint32_t src = __shfl_sync(0xffffffffu, cl, i);
+                    const float4 *y =
+                        reinterpret_cast<const float4 *>(ycol + static_cast<size_t>(src) * a.kp);
+#pragma unroll
+                    for (int h = 0; h < H; ++h)
+                        add4(acc[h], __ldg(y + h));
+                }
             }
-            const uint32_t r = a.n_long + (v - a.n_chunks);
-            const float deg = static_cast<float>(dc);
+            if (!on)
+                continue;
 #pragma unroll
             for (int h = 0; h < H; ++h) {
-                const float y[4] = {yo[h].x, yo[h].y, yo[h].z, yo[h].w};
-                float yn[4];
-#pragma unroll
-                for (int c = 0; c < 4; ++c)
-                    yn[c] = finish_column(a, r, dc, deg, dampf, omd, acc[h][c], y[c], act[h][c],
-                                          sc[h][c], seed[h][c], res[h][c], sink[h][c]);
-                if (on[h])
-                    *reinterpret_cast<float4 *>(a.y_out + static_cast<size_t>(r) * a.kp + h * 128 +
-                                                lane * 4) = make_float4(yn[0], yn[1], yn[2], yn[3]);
+                if (v < a.n_chunks)
+                    *reinterpret_cast<float4 *>(a.chunk_val + static_cast<size_t>(v) * a.kp + col +
+                                                4 * h) =
+                        make_float4(acc[h][0], acc[h][1], acc[h][2], acc[h][3]);
+                else
+                    finish(a, col + 4 * h, a.n_long + (v - a.n_chunks), acc[h], res[h], sink + 4 * h);
             }
-        };
-        open_row();
-        while (k < q.end) {
-            if (!bar_wait(q.bar + cur, (q.phases >> cur) & 1)) {
-                ok = false;
-                break;
-            }
-            q.phases ^= 1u << cur;
-            const uint32_t n = min(kBulkArcs, q.end - k);
-            const unsigned char *st = q.rows + cur * kBulkArcs * q.row_bytes + lane * 16;
-            for (uint32_t i = 0; i < n; ++i, ++k) {
-                while (k == e) {
-                    close_row();
-                    ++v;
-                    e = __ldg(a.vrange + v).y;
-                    open_row();
-                }
-#pragma unroll
-                for (int h = 0; h < H; ++h)
-                    if (on[h])
-                        add4(acc[h], *reinterpret_cast<const float4 *>(st + i * q.row_bytes + h * 512));
-            }
-            __syncwarp();  // every lane has read the stage
-            cur = cur + 1 == stages ? 0 : cur + 1;
-            ring_issue(a, q);
         }
-        if (!ok)
-            break;
-        for (;;) {  // the last row with arcs and the empty rows behind it
-            close_row();
-            if (++v >= v_end)
-                break;
-            open_row();
-        }
-    }
-    if (!ok) {
-        // A copy never arrived: report it, and give the others their time.
-        if (lane == 0)
-            a.st->error = 1;
-        for (uint32_t i = 0; i < stages; ++i)
-            bar_wait(q.bar + i, (q.phases >> i) & 1);
     }
     // Per-column sums over the warps (column_partials).
-    double *s_buf = reinterpret_cast<double *>(s_ring);
     for (int pass = 0; pass < 2; ++pass) {
-        __syncthreads();
+        if (pass == 1) {
+            __syncthreads();
+            if (on)
 #pragma unroll
-        for (int h = 0; h < H; ++h)
-            if (on[h])
+                for (int h = 0; h < H; ++h)
 #pragma unroll
-                for (int c = 0; c < 4; ++c)
-                    s_buf[wid * a.kp + h * 128 + lane * 4 + c] = pass == 0 ? res[h][c] : sink[h][c];
+                    for (int c = 0; c < 4; ++c)
+                        sink[4 * h + c] = res[h][c];
+        }
         __syncthreads();
-        for (uint32_t col = threadIdx.x; col < a.kp; col += kBulkThreads) {
+        for (uint32_t k = threadIdx.x; k < a.kp; k += kPprThreads) {
             double sum = 0.0;
-            for (uint32_t w = 0; w < kBulkWarps; ++w)
-                sum += s_buf[w * a.kp + col];
-            (pass == 0 ? a.cta_res : a.cta_sink)[static_cast<size_t>(blockIdx.x) * a.kp + col] = sum;
+            for (uint32_t w = 0; w < kPprWarps; ++w)
+                sum += s_buf[w * a.kp + k];
+            (pass == 0 ? a.cta_sink : a.cta_res)[static_cast<size_t>(blockIdx.x) * a.kp + k] = sum;
         }
     }
 }
@@ -447,7 +318,6 @@ __global__ void __launch_bounds__(kPprThreads, 4) ppr_sweep(PprArgs a) {
     extern __shared__ double s_buf[];
     if (*(volatile int *)&a.st->all_done)
         return;
-    const uint32_t lane = threadIdx.x & 31;
     const PprLane L = ppr_lane(a);
     double res[4], sink[4];
 #pragma unroll
@@ -470,7 +340,7 @@ __global__ void __launch_bounds__(kPprThreads, 4) ppr_sweep(PprArgs a) {
                     *reinterpret_cast<float4 *>(a.chunk_val + static_cast<size_t>(v) * a.kp + L.col) =
                         make_float4(acc[0], acc[1], acc[2], acc[3]);
                 else
-                    finish(a, L, a.n_long + (v - a.n_chunks), acc, res, sink);
+                    finish(a, L.col, a.n_long + (v - a.n_chunks), acc, res, sink);
             }
             cur = nxt;
         }
@@ -506,7 +376,7 @@ __global__ void __launch_bounds__(kPprThreads) ppr_fixup(PprArgs a, double *fix_
 #pragma unroll 8
         for (uint32_t k = a.chunk_begin[r]; k < ke; ++k)
             add4(acc, *reinterpret_cast<const float4 *>(a.chunk_val + static_cast<size_t>(k) * a.kp + L.col));
-        finish(a, L, r, acc, res, sink);
+        finish(a, L.col, r, acc, res, sink);
     }
     column_partials(a, L, 1, res, sink, s_buf, fix_res, fix_sink, a.cta_res, a.cta_sink,
                     a.sweep_ctas);
@@ -743,23 +613,15 @@ void run_ppr(nkg_graph *g, const nkg_pr_params &p, uint32_t k, const uint32_t *s
         ppr_chunk_rows<<<sms * 4, 256, 0, s>>>(chunk_begin, n_long, chunk_row.get());
     int occ = 0;
     const size_t smem_sweep = static_cast<size_t>(kPprWarps) * 128 * sizeof(double);
-    // Wide rows: one CTA per SM, as many stages per warp as fit.
-    const bool wide = parts == 2;
-    const size_t stage_bytes = static_cast<size_t>(kBulkWarps) * kBulkArcs * kp * sizeof(float);
-    const uint32_t stages = static_cast<uint32_t>(
-        std::min<size_t>(kBulkStages, kBulkBytes / stage_bytes));
-    const size_t smem_bulk = stages * stage_bytes;
-    if (wide)  // the kernel's own most, not this call's: other handles launch it too
-        NKG_CUDA(cudaFuncSetAttribute(ppr_sweep_bulk, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      static_cast<int>(kBulkBytes)));
-    NKG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, ppr_sweep, kPprThreads,
-                                                           smem_sweep));
-    occ = wide ? 1 : std::max(occ, 1);
-    const uint32_t warps = wide ? kBulkWarps : kPprWarps;  // per CTA
+    // More than 64 columns: one arc per warp and step (ppr_sweep_one).
+    const auto sweep = groups > 1 ? ppr_sweep : parts == 1 ? ppr_sweep_one<1> : ppr_sweep_one<2>;
+    NKG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, sweep, kPprThreads,
+                                                           smem_sweep * parts));
+    occ = std::max(occ, 1);
     const uint32_t sweep_ctas = static_cast<uint32_t>(std::max<uint64_t>(
-        1, std::min<uint64_t>(static_cast<uint64_t>(occ) * sms, (nv + warps - 1) / warps)));
+        1, std::min<uint64_t>(static_cast<uint64_t>(occ) * sms, (nv + kPprWarps - 1) / kPprWarps)));
     const uint32_t units = std::max<uint32_t>(
-        1, std::min<uint32_t>(sweep_ctas * warps * 4, std::max<uint32_t>(nv, 1)));
+        1, std::min<uint32_t>(sweep_ctas * kPprWarps * 4, std::max<uint32_t>(nv, 1)));
     DeviceArray<uint64_t> cost(std::max<uint32_t>(nv, 1)), cost_incl(std::max<uint32_t>(nv, 1));
     DeviceArray<uint32_t> unit_start(units + 1);
     DeviceArray<uint2> vrange(std::max<uint32_t>(nv, 1));
@@ -846,17 +708,12 @@ void run_ppr(nkg_graph *g, const nkg_pr_params &p, uint32_t k, const uint32_t *s
         for (int i = 0; i < 8; ++i) {
             a.y_in = ((it + i) & 1) ? y1.get() : y0.get();
             a.y_out = ((it + i) & 1) ? y0.get() : y1.get();
-            if (wide)
-                ppr_sweep_bulk<<<sweep_ctas, kBulkThreads, smem_bulk, s>>>(a, stages);
-            else
-                ppr_sweep<<<sweep_ctas, kPprThreads, smem_sweep, s>>>(a);
+            sweep<<<sweep_ctas, kPprThreads, smem_sweep * parts, s>>>(a);
             ppr_fixup<<<fix_ctas, kPprThreads, smem_sweep, s>>>(a, fix_res.get(), fix_sink.get());
         }
         launches += 16;
         NKG_CUDA(cudaGetLastError());
         h = read_scalar(st.get(), s);
-        if (h.error)
-            throw Error(NKG_ERR_TIMEOUT, "a row copy of the personalised PageRank sweep timed out");
         if (h.all_done)
             break;
         check_cancel(g, "personalised PageRank run cancelled");

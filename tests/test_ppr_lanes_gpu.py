@@ -1,5 +1,6 @@
 """Personalised PageRank columns for every way a row's columns are laid over
-the lanes of a warp: one to 32 lanes, one or two parts, several groups."""
+the lanes of a warp: one to 32 lanes, several groups of lanes on different arcs (up to 64
+columns), one arc per warp with 4 or 8 columns a lane (more)."""
 import numpy as np
 import pytest
 
