@@ -516,7 +516,11 @@ __global__ void ppr_vrow_ranges(const uint32_t *__restrict__ row_ptr,
         e = row_ptr[r + 1];
     }
     range[v] = make_uint2(b, e);
-    cost[v] = static_cast<uint64_t>(e - b) + 4;  // arcs + the row's epilogue
+    // Arcs, and eight arcs' time for the row's end. With four, the rows without
+    // arcs, which are last in the order, made the last units the longest: R-MAT
+    // 20, 16 sweeps, 4 / 8 / 16 arcs: 37 columns 15.1 / 13.5 / 12.9 ms, 64 16.4 /
+    // 14.6 / 14.7, 256 47.2 / 41.4 / 42.9.
+    cost[v] = static_cast<uint64_t>(e - b) + 8;
 }
 
 __global__ void ppr_unit_bounds(const uint64_t *__restrict__ cost_incl, uint32_t nv, uint32_t units,
