@@ -210,12 +210,14 @@ __global__ void validate_and_count(const uint64_t *__restrict__ in_ptr,
 }
 
 // Sort key per original id: deleted nodes 0 (sorted last), existing nodes
-// in-degree + 1 with, below it, the bit length of the out-degree, so that the
-// nodes of one in-degree are ordered by how often they are gathered (sinks,
-// never gathered, last): gathers of the many low in-degree nodes then share
-// lines. With `bucketed` degree_bucket(in-degree) + 1 (the stable sort then
-// keeps the caller's order inside a bucket). Counts sinks (existing,
-// out-degree 0).
+// in-degree + 1 with, below it, whether there are out-arcs: sinks, which are
+// never gathered, come last among the nodes of one in-degree, so that gathers of
+// the many low in-degree nodes share lines. 20 iterations, FP64, without / with:
+// R-MAT 24 14.19 / 13.95 ms, R-MAT 23 8.16 / 8.10, R-MAT 20 1.54 / 1.51. (By the
+// bit length of the out-degree: 13.98, 8.18 and 1.52, but ids that carry
+// locality lose it: 4M nodes, arcs within 50 ids, 8.39 against 7.68.) With
+// `bucketed` degree_bucket(in-degree) + 1 (the stable sort then keeps the
+// caller's order inside a bucket). Counts sinks (existing, out-degree 0).
 __global__ void make_keys(const uint64_t *__restrict__ in_ptr, const uint32_t *__restrict__ outdeg,
                           const uint8_t *__restrict__ exists, uint64_t z, int bucketed,
                           uint32_t *__restrict__ keys, uint32_t *__restrict__ ids,
@@ -227,8 +229,8 @@ __global__ void make_keys(const uint64_t *__restrict__ in_ptr, const uint32_t *_
         const uint64_t d = in_ptr[i + 1] - in_ptr[i];
         const uint32_t o = outdeg[i];
         uint32_t k = degree_bucket(static_cast<uint32_t>(d)) + 1;
-        if (!bucketed)  // 27 bits of in-degree (more is one class: all hubs), 5 of out-degree
-            k = (min(static_cast<uint32_t>(d), (1u << 27) - 2) + 1) << 5 | min(32u - __clz(o), 31u);
+        if (!bucketed)  // in-degrees from 2^31 - 2 on are one class
+            k = (static_cast<uint32_t>(d < (1u << 31) - 2 ? d : (1u << 31) - 2) + 1) << 1 | (o ? 1u : 0u);
         keys[i] = ex ? k : 0u;
         ids[i] = static_cast<uint32_t>(i);
         sink = ex && o == 0;
