@@ -535,8 +535,9 @@ __device__ __forceinline__ V lane_chunk_sum(const V *__restrict__ v, uint32_t cb
 // Calls finish(r, sum) once for every split row r < n_long with the sum of its
 // chunk sums, in a fixed order: a warp for each of the first n_vlong rows
 // (lane-strided partials in V, then across lanes in double), row_lanes() lanes
-// for each other (four loads of a lane in flight; one thread per row took 42
-// us of every R-MAT 24 iteration where source blocks give a row a dozen sums).
+// for each other, in double too (four loads of a lane in flight; one thread per
+// row took 42 us of every R-MAT 24 iteration where source blocks give a row a
+// dozen sums).
 // Every thread of the CTA calls it.
 template <int THREADS, typename V, typename F>
 __device__ __forceinline__ void for_split_rows(const uint32_t *__restrict__ chunk_begin,
@@ -563,7 +564,7 @@ __device__ __forceinline__ void for_split_rows(const uint32_t *__restrict__ chun
          base < n_long; base += stride) {
         const uint32_t r = base + (lane >> shift);
         const uint32_t e = r < n_long ? chunk_begin[r + 1] : 0u;
-        V sum = V(0);
+        double sum = 0.0;
         for (uint32_t k = r < n_long ? chunk_begin[r] + sub : 0u; k < e; k += 4 * lanes) {
             V x[4];
 #pragma unroll
@@ -571,13 +572,13 @@ __device__ __forceinline__ void for_split_rows(const uint32_t *__restrict__ chun
                 x[q] = k + q * lanes < e ? chunk_val[k + q * lanes] : V(0);
 #pragma unroll
             for (uint32_t q = 0; q < 4; ++q)
-                sum += x[q];
+                sum += static_cast<double>(x[q]);
         }
         __syncwarp();
         for (uint32_t o = lanes / 2; o > 0; o >>= 1)
             sum += __shfl_xor_sync(0xffffffffu, sum, o);
         if (sub == 0 && r < n_long)
-            finish(r, sum);
+            finish(r, static_cast<V>(sum));
     }
 }
 

@@ -43,6 +43,23 @@ def test_blocked_sweeps_match_oracle(oracle_mod, rmat, norm, distribute):
         assert np.abs(s - o.scores).sum() <= 2e-9
 
 
+def test_fp32_rows_of_many_segments_round_like_their_epilogue(rmat):
+    """Rows of 17 to 128 chunk sums: added in FP32 (four lanes, then across them)
+    the sums cost 0.91 in the unit below. Left are the chunks' own sums, whose
+    errors average out over dozens of chunks, and the four roundings of a row's
+    epilogue and output, each uniform in one unit times a mantissa of 0.72 on
+    average: sqrt(4 / 3) * 0.72."""
+    csr, dg = rmat
+    rows = np.diff(csr.in_ptr.astype(np.int64))
+    rows = (rows >= 8000) & (rows < 16000)
+    assert rows.sum() > 200
+    s32, s64 = (dg.run(dg.params(0.85, 0.0, 0, False, False, prec, 5))[0]
+                for prec in (_capi.NKG_PREC_FP32, _capi.NKG_PREC_FP64))
+    rel = (s32 / s64 - 1) * 2.0 ** 24
+    rel = rel[rows] - np.median(rel)  # the normalisation's factor is every row's
+    assert np.sqrt((rel * rel).mean()) <= np.sqrt(4 / 3) * 0.72
+
+
 def test_blocked_centralities_match_oracle(oracle_mod, rmat):
     csr, dg = rmat
     s, it, _ = dg.eigenvector(1e-9)
