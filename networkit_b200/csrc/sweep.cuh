@@ -509,35 +509,41 @@ inline unsigned split_fix_ctas(uint32_t n_long, uint32_t n_vlong, uint32_t n_hot
         1, (n_vlong + w - 1) / w + std::min<uint64_t>(n_hot ? 592 : 1184, (short_rows + rows - 1) / rows)));
 }
 
-// Lane-strided partial sum of one split row's chunk partials
-// v[cb + lane], v[cb + lane + 32], ... in ascending order, with 16 loads in
-// flight at a time (a row has up to about a thousand chunks). Absent entries
-// add zero, so the sum equals the one-at-a-time loop bit for bit.
-template <typename V>
-__device__ __forceinline__ V lane_chunk_sum(const V *__restrict__ v, uint32_t cb, uint32_t ce,
-                                            int lane) {
+// Sum of one split row's chunk sums v[first], v[first + STEP], ... before ce,
+// in double and in that order, with 16 loads in flight at a time.
+template <uint32_t STEP, typename V>
+__device__ __forceinline__ double strided_chunk_sum(const V *__restrict__ v, uint32_t first,
+                                                    uint32_t ce) {
     constexpr int kBatch = 16;
-    V part = V(0);
-    for (uint32_t k0 = cb + lane; k0 < ce; k0 += 32 * kBatch) {
+    double part = 0.0;
+    for (uint32_t k0 = first; k0 < ce; k0 += STEP * kBatch) {
         V x[kBatch];
 #pragma unroll
         for (int q = 0; q < kBatch; ++q) {
-            const uint32_t k = k0 + 32u * q;
+            const uint32_t k = k0 + STEP * q;
             x[q] = k < ce ? v[k] : V(0);
         }
 #pragma unroll
         for (int q = 0; q < kBatch; ++q)
-            part += x[q];
+            part += static_cast<double>(x[q]);
     }
     return part;
 }
 
+// Rows of more chunk sums than this are summed by a whole CTA where it has no
+// more than kCtaRows of them: a warp adds about 800 sums a microsecond, so a row
+// of 8M arcs (125,000 chunks of 64) held an iteration up for 0.15 ms, but eight
+// rows of 5,000 sums one after the other take a CTA 20 us and its eight warps 7.
+// 40 iterations of 4M arcs and one row of 2M more, FP64, a warp / a CTA: 3.7 /
+// 2.4 ms; of 8M more 10.2 / 4.2.
+constexpr uint32_t kCtaSums = 2048;
+constexpr uint32_t kCtaRows = 2;
+
 // Calls finish(r, sum) once for every split row r < n_long with the sum of its
-// chunk sums, in a fixed order: a warp for each of the first n_vlong rows
-// (lane-strided partials in V, then across lanes in double), row_lanes() lanes
-// for each other, in double too (four loads of a lane in flight; one thread per
-// row took 42 us of every R-MAT 24 iteration where source blocks give a row a
-// dozen sums).
+// chunk sums, in double and in a fixed order: a warp, or a CTA (kCtaSums),
+// for each of the first n_vlong rows, row_lanes() lanes for each other (four
+// loads of a lane in flight; one thread per row took 42 us of every R-MAT 24
+// iteration where source blocks give a row a dozen sums).
 // Every thread of the CTA calls it.
 template <int THREADS, typename V, typename F>
 __device__ __forceinline__ void for_split_rows(const uint32_t *__restrict__ chunk_begin,
@@ -548,14 +554,28 @@ __device__ __forceinline__ void for_split_rows(const uint32_t *__restrict__ chun
     const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const uint32_t vctas = (n_vlong + w - 1) / w;
     if (blockIdx.x < vctas) {
-        const uint32_t r = blockIdx.x * w + wid;
-        if (r >= n_vlong)
+        __shared__ double s_part[32];
+        // Rows blockIdx.x, + vctas, ...: the longest rows, which are first, go to
+        // CTAs of their own.
+        const uint32_t r = blockIdx.x + wid * vctas;
+        const uint32_t b = r < n_vlong ? chunk_begin[r] : 0u;
+        const uint32_t e = r < n_vlong ? chunk_begin[r + 1] : 0u;
+        const int many = __syncthreads_count(lane == 0 && e - b > kCtaSums);
+        const bool cta_rows = many > 0 && many <= static_cast<int>(kCtaRows);
+        for (uint32_t q = blockIdx.x; cta_rows && q < n_vlong; q += vctas) {
+            const uint32_t qb = chunk_begin[q], qe = chunk_begin[q + 1];
+            if (qe - qb <= kCtaSums)
+                continue;
+            const double sum = block_sum<THREADS>(
+                strided_chunk_sum<THREADS>(chunk_val, qb + threadIdx.x, qe), s_part);
+            if (threadIdx.x == 0)
+                finish(q, static_cast<V>(sum));
+        }
+        if (r >= n_vlong || (cta_rows && e - b > kCtaSums))
             return;
-        const V part = lane_chunk_sum(chunk_val, chunk_begin[r], chunk_begin[r + 1],
-                                      static_cast<int>(lane));
-        const V acc = static_cast<V>(warp_sum(static_cast<double>(part)));
+        const double sum = warp_sum(strided_chunk_sum<32>(chunk_val, b + lane, e));
         if (lane == 0)
-            finish(r, acc);
+            finish(r, static_cast<V>(sum));
         return;
     }
     const uint32_t sub = lane & (lanes - 1);
