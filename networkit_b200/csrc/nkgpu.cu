@@ -210,16 +210,19 @@ __global__ void validate_and_count(const uint64_t *__restrict__ in_ptr,
 }
 
 // Sort key per original id: deleted nodes 0 (sorted last), existing nodes
-// in-degree + 1 with, below it, whether there are out-arcs: sinks, which are
-// never gathered, come last among the nodes of one in-degree, so that gathers of
-// the many low in-degree nodes share lines. 20 iterations, FP64, without / with:
-// R-MAT 24 14.19 / 13.95 ms, R-MAT 23 8.16 / 8.10, R-MAT 20 1.54 / 1.51. (By the
-// bit length of the out-degree: 13.98, 8.18 and 1.52, but ids that carry
-// locality lose it: 4M nodes, arcs within 50 ids, 8.39 against 7.68.) With
-// `bucketed` degree_bucket(in-degree) + 1 (the stable sort then keeps the
-// caller's order inside a bucket). Counts sinks (existing, out-degree 0).
+// in-degree + 1 and, below it, how much they are gathered, so that the gathers
+// of the many low in-degree nodes share lines (the stable sort keeps the
+// caller's order among equals). kRowsByUse: the bit length of the out-degree;
+// kRowsByDegree, which a caller may ask for whatever its ids are: only whether
+// there are out-arcs (sinks, never gathered, last), as more would take neighbours
+// apart where ids carry locality (4M nodes, arcs within 50 ids, 20 FP64
+// iterations 8.39 ms by use, 7.68 sinks last, 7.68 neither). Neither / sinks last
+// / by use, ms: R-MAT 24 14.19 / 13.95 / 13.98, R-MAT 20 1.54 / 1.51 / 1.52, 20M
+// nodes and 40M random arcs 11.1 / 10.4 / 9.9. kRowsBucketed:
+// degree_bucket(in-degree) + 1. Counts sinks (existing, out-degree 0).
+enum RowKeys { kRowsByDegree = 0, kRowsBucketed = 1, kRowsByUse = 2 };
 __global__ void make_keys(const uint64_t *__restrict__ in_ptr, const uint32_t *__restrict__ outdeg,
-                          const uint8_t *__restrict__ exists, uint64_t z, int bucketed,
+                          const uint8_t *__restrict__ exists, uint64_t z, int order,
                           uint32_t *__restrict__ keys, uint32_t *__restrict__ ids,
                           unsigned long long *__restrict__ sinks) {
     const uint64_t i = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x;
@@ -229,8 +232,11 @@ __global__ void make_keys(const uint64_t *__restrict__ in_ptr, const uint32_t *_
         const uint64_t d = in_ptr[i + 1] - in_ptr[i];
         const uint32_t o = outdeg[i];
         uint32_t k = degree_bucket(static_cast<uint32_t>(d)) + 1;
-        if (!bucketed)  // in-degrees from 2^31 - 2 on are one class
-            k = (static_cast<uint32_t>(d < (1u << 31) - 2 ? d : (1u << 31) - 2) + 1) << 1 | (o ? 1u : 0u);
+        if (order != kRowsBucketed) {  // in-degrees from 2^27 - 2 on are one class
+            const uint32_t c = d < (1u << 27) - 2 ? static_cast<uint32_t>(d) : (1u << 27) - 2;
+            const uint32_t use = order == kRowsByUse ? min(32u - __clz(o), 31u) : o ? 1u : 0u;
+            k = (c + 1) << 5 | use;
+        }
         keys[i] = ex ? k : 0u;
         ids[i] = static_cast<uint32_t>(i);
         sink = ex && o == 0;
@@ -1573,8 +1579,9 @@ static nkg_graph *build_graph(std::unique_ptr<nkg_graph> g, DeviceArray<uint64_t
     // Relabelling order: in-degree descending (row_order 0) or half-octave
     // in-degree buckets descending (row_order 1), ties by id; -1 picks 1 when
     // the caller's ids carry locality (more than 1/4 of 65,536 sampled arcs
-    // join ids closer than max(64, z/1024)).
+    // join ids closer than max(64, z/1024)), and otherwise 0 by use.
     int row_order = opt ? opt->row_order : -1;  // no options: automatic
+    const bool automatic = row_order < 0;
     require(row_order >= -1 && row_order <= 1, "row_order must be -1, 0 or 1");
     if (row_order < 0) {
         constexpr uint32_t kSamples = 65536;
@@ -1589,7 +1596,8 @@ static nkg_graph *build_graph(std::unique_ptr<nkg_graph> g, DeviceArray<uint64_t
     g->row_order = row_order;
     DeviceArray<uint32_t> keys(z), ids(z), keys_s(z), ids_s(z);
     make_keys<<<ceil_div(z, 256), 256, 0, s>>>(d_ptr.get(), outdeg.get(), d_ex.get(), z,
-                                               row_order, keys.get(), ids.get(), cnt.get());
+                                               automatic && !row_order ? kRowsByUse : row_order,
+                                               keys.get(), ids.get(), cnt.get());
     NKG_CUDA(cudaGetLastError());
     size_t tmp_bytes = 0;
     NKG_CUDA(cub::DeviceRadixSort::SortPairsDescending(nullptr, tmp_bytes, keys.get(), keys_s.get(),
