@@ -36,7 +36,8 @@ struct RefineWork {
 // Buffers of the one-launch run of a small graph (small.cuh), kept between runs.
 struct SmallWork {
     SmallPlan plan{};
-    unsigned ctas = 0;  // 0: not set up
+    unsigned ctas = 0;     // 0: not set up
+    bool declined = false; // this graph's runs are captured sweeps
     DeviceArray<double> y0, y1, part;
     DeviceArray<SmallState> st;
     PinnedHost<SmallState> host;

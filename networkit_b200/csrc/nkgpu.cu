@@ -2220,14 +2220,13 @@ static bool runs_small(const nkg_graph *g) {
 }
 
 // Class boundaries of the rows: how many are longer than each threshold (a
-// prefix of the rows, thresholds being powers of two). One thread each.
-__global__ void small_bounds(const uint32_t *__restrict__ row_ptr, uint32_t n,
+// prefix of the rows, thresholds being powers of two), one thread each, and
+// the hub arcs of the first of `ctas` CTAs, whose hubs are the longest. One warp.
+__global__ void small_bounds(const uint32_t *__restrict__ row_ptr, uint32_t n, uint32_t ctas,
                              uint32_t *__restrict__ bounds) {
     const uint32_t len[kSmallClasses] = {kSmallHub, 16 * kSmallBatch, 8 * kSmallBatch,
                                          4 * kSmallBatch, 2 * kSmallBatch, kSmallBatch};
-    if (threadIdx.x >= kSmallClasses)
-        return;
-    uint32_t lo = 0, hi = n;
+    uint32_t lo = 0, hi = threadIdx.x < kSmallClasses ? n : 0;
     while (lo < hi) {
         const uint32_t mid = (lo + hi) >> 1;
         if (row_ptr[mid + 1] - row_ptr[mid] > len[threadIdx.x])
@@ -2235,21 +2234,34 @@ __global__ void small_bounds(const uint32_t *__restrict__ row_ptr, uint32_t n,
         else
             hi = mid;
     }
-    bounds[threadIdx.x] = lo;
+    if (threadIdx.x < kSmallClasses)
+        bounds[threadIdx.x] = lo;
+    const uint32_t hubs = __shfl_sync(0xffffffffu, lo, 0);
+    uint32_t arcs = 0;
+    for (uint64_t h = static_cast<uint64_t>(threadIdx.x) * ctas; h < hubs; h += 32ull * ctas)
+        arcs += row_ptr[h + 1] - row_ptr[h];
+    arcs = __reduce_add_sync(0xffffffffu, arcs);
+    if (threadIdx.x == 0)
+        bounds[kSmallClasses] = arcs;
 }
 
 static void small_setup(nkg_graph *g) {
     SmallWork &W = g->small;
-    if (W.ctas)
+    if (W.ctas || W.declined)
         return;
     cudaStream_t s = g->stream;
     const uint32_t n = static_cast<uint32_t>(g->n);
-    DeviceArray<uint32_t> bounds(kSmallClasses);
-    small_bounds<<<1, 32, 0, s>>>(g->row_ptr.get(), n, bounds.get());
+    const unsigned sms = num_sms(g->device);
+    DeviceArray<uint32_t> bounds(kSmallClasses + 1);
+    small_bounds<<<1, 32, 0, s>>>(g->row_ptr.get(), n, sms, bounds.get());
     NKG_CUDA(cudaGetLastError());
-    uint32_t h[kSmallClasses];
+    uint32_t h[kSmallClasses + 1];
     NKG_CUDA(cudaMemcpyAsync(h, bounds.get(), sizeof(h), cudaMemcpyDeviceToHost, s));
     NKG_CUDA(cudaStreamSynchronize(s));
+    if (h[kSmallClasses] > kSmallHubArcs + g->arcs / (2 * sms)) {
+        W.declined = true;
+        return;
+    }
     SmallPlan &P = W.plan;
     P.row[0] = 0;
     std::copy(h, h + kSmallClasses, P.row + 1);
@@ -2259,8 +2271,7 @@ static void small_setup(nkg_graph *g) {
         P.task[c + 1] = P.task[c] + ceil_div(P.row[c + 2] - P.row[c + 1], 1u << c);
     // One CTA per SM, fewer where each would have less than four warps' tasks.
     const unsigned ctas = std::max<unsigned>(
-        1, std::min<unsigned>(num_sms(g->device),
-                              std::max<unsigned>(ceil_div(P.task[kSmallClasses], 4), P.row[1])));
+        1, std::min<unsigned>(sms, std::max<unsigned>(ceil_div(P.task[kSmallClasses], 4), P.row[1])));
     W.y0.alloc(n);
     W.y1.alloc(n);
     W.part.alloc(7 * static_cast<size_t>(ctas));
@@ -2273,7 +2284,6 @@ template <typename T>
 static RunResult run_small(nkg_graph *g, const nkg_pr_params &p, const double *d_tele,
                            double *d_out) {
     cudaStream_t s = g->stream;
-    small_setup(g);
     SmallWork &W = g->small;
     Plane<T> &P = plane<T>(g);
     const uint32_t n = static_cast<uint32_t>(g->n);
@@ -2306,6 +2316,7 @@ static RunResult run_small(nkg_graph *g, const nkg_pr_params &p, const double *d
     a.z = g->z;
     a.n = n;
     a.cap = kSmallSweeps;
+    a.polls = kSmallPolls;
     a.normalized = p.normalized ? 1 : 0;
     const double S0 = static_cast<double>(g->sinks) * a.rp.inv_n;
     a.coef0 = p.distribute_sinks ? (d_tele ? S0 : S0 / static_cast<double>(n)) : 0.0;
@@ -2343,8 +2354,11 @@ static RunResult run_small(nkg_graph *g, const nkg_pr_params &p, const double *d
 template <typename T, bool WEIGHTED>
 static RunResult run_power(nkg_graph *g, const nkg_pr_params &p, const double *d_tele,
                            double *d_out) {
-    if (!WEIGHTED && runs_small(g))
-        return run_small<T>(g, p, d_tele, d_out);
+    if (!WEIGHTED && runs_small(g)) {
+        small_setup(g);
+        if (g->small.ctas)
+            return run_small<T>(g, p, d_tele, d_out);
+    }
     cudaStream_t s = g->stream;
     sweep_setup<T, WEIGHTED>(g);
     Plane<T> &P = plane<T>(g);

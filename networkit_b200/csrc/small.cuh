@@ -46,6 +46,15 @@ struct SmallPlan {
     uint32_t task[kSmallClasses + 1];
 };
 
+// A hub is one CTA's work and the others wait for it, so graphs with longer rows
+// than this stay with the captured sweeps, which cut them into chunks for all
+// SMs: hub arcs of the CTA that has most, beyond half a CTA's share of all arcs
+// (by which the captured sweeps are slower elsewhere). 40 FP64 sweeps of M arcs
+// and one row of H more, one launch / captured, ms: M 0.3M, H 8k 0.40 / 0.69,
+// 32k 0.59 / 0.69, 128k 1.38 / 0.78, 8M 65 / 2.5; M 4M, H 32k 1.60 / 1.71, 128k
+// 3.56 / 1.79, 8M 164 / 4.1; M 12M, H 32k 3.05 / 3.85, 128k 5.06 / 3.94.
+constexpr uint32_t kSmallHubArcs = 28672;
+
 // Device state of a run, and what the host reads back.
 struct SmallState {
     unsigned long long iteration;
@@ -69,6 +78,7 @@ struct SmallArgs {
     uint64_t z;
     uint32_t n, trace_cap;
     uint32_t cap;        // sweeps of this launch
+    uint32_t polls;      // of the grid barrier before it gives up
     int first, normalized;
     double coef0;        // sink term of the first sweep
 };
@@ -87,17 +97,16 @@ __device__ __forceinline__ float ld_y(const float *p) {
 
 // All CTAs of the launch arrive, then go on; the writes before it are visible
 // after it. False once the wait ran out (every CTA then gives up the same way).
-__device__ __forceinline__ bool small_barrier(SmallState *st, unsigned int &target, bool *s_ok) {
+__device__ __forceinline__ bool small_barrier(SmallState *st, uint32_t polls, unsigned int &target,
+                                              bool *s_ok) {
     __syncthreads();
     if (threadIdx.x == 0) {
         target += gridDim.x;
         __threadfence();
         atomicAdd(&st->barrier, 1u);
-        uint32_t polls = 0;
-        unsigned int v;
-        do {
+        unsigned int v = 0;
+        for (uint32_t i = 0; v < target && i < polls; ++i)
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(&st->barrier) : "memory");
-        } while (v < target && ++polls < kSmallPolls);
         if (v < target)
             st->error = 1;
         *s_ok = v >= target;
@@ -233,7 +242,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) small_kernel(SmallArgs<T> a)
             const uint32_t dc = a.degc[r];
             a.y0[r] = dc == 0 ? x0 : x0 / static_cast<T>(dc);
         }
-        if (!small_barrier(a.st, target, &s_ok))
+        if (!small_barrier(a.st, a.polls, target, &s_ok))
             return;
     } else {
         __syncthreads();
@@ -327,7 +336,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) small_kernel(SmallArgs<T> a)
             }
         }
         ++it;
-        if (!small_barrier(a.st, target, &s_ok))
+        if (!small_barrier(a.st, a.polls, target, &s_ok))
             return;
     }
     if (gid == 0) {
@@ -372,7 +381,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) small_kernel(SmallArgs<T> a)
             pf[2 * nctas + blockIdx.x] = mx;
         }
     }
-    if (!small_barrier(a.st, target, &s_ok))
+    if (!small_barrier(a.st, a.polls, target, &s_ok))
         return;
     if (wid == 0) {
         s = ss = 0.0;

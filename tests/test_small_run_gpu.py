@@ -32,6 +32,8 @@ GRAPHS = {
     # one batch of 8 arcs a lane: each class at its first and last length
     "classes": lambda: graph_of_rows([1, 7, 8, 9, 16, 17, 32, 33, 64, 65, 128, 129, 256, 257] * 9,
                                      700, 1),
+    # rows of a whole CTA: up to what one launch takes, and one longer (captured sweeps)
+    "hub_rows": lambda: graph_of_rows([2047, 2048, 2049, 9000, 28000, 1, 0, 3], 3000, 2),
     "hubs": lambda: graph_of_rows([2047, 2048, 2049, 9000, 70000, 1, 0, 3], 3000, 2),
     "one_node": lambda: in_csr_from_edges(1, [], [], directed=True),
     "self_loop": lambda: in_csr_from_edges(1, [0], [0], directed=True),
@@ -97,3 +99,20 @@ def test_small_run_with_deleted_nodes(oracle_mod):
     s, it, _, _ = dg.run(p)
     o = oracle_mod.pagerank(csr, tol=1e-12, norm=0, distribute_sinks=True)
     assert abs(it - o.iterations) <= 1 and np.abs(s - o.scores).sum() <= 1e-11
+
+
+@pytest.mark.parametrize("hub,one_launch", [(28_672, True), (28_900, False), (1_000_000, False)])
+def test_a_row_longer_than_a_ctas_share_is_cut_into_chunks(oracle_mod, hub, one_launch):
+    """One CTA adds up a row in the one-launch run, so a graph with a longer row
+    than 28,672 arcs and half an SM's share takes the captured sweeps."""
+    csr = graph_of_rows([hub, 3000, 7, 0, 2], 5000, 11)
+    assert 28_672 + csr.arcs // 200 < 28_900 or hub > 100_000  # at least 100 SMs
+    dg = _capi.DeviceGraph(csr)
+    o = oracle_mod.pagerank(csr, tol=1e-11, norm=0, distribute_sinks=True)
+    p = dg.params(0.85, 1e-11, 0, False, True, _capi.NKG_PREC_FP64, 5000)
+    s, it, _, st = dg.run(p)
+    assert (st["kernel_launches"] == 1) == one_launch
+    assert abs(it - o.iterations) <= 1 and np.abs(s - o.scores).sum() <= 1e-11
+    p32 = dg.params(0.85, 0.0, 0, False, True, _capi.NKG_PREC_FP32, 60)
+    # FP32 scores of unit mass, one of them most of it: a few roundings of 2^-24
+    assert np.abs(dg.run(p32)[0] - o.scores).sum() <= 1e-6
