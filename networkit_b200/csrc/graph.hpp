@@ -38,6 +38,8 @@ struct SmallWork {
     SmallPlan plan{};
     unsigned ctas = 0;     // 0: not set up
     bool declined = false; // this graph's runs are captured sweeps
+    uint32_t polls = kSmallPolls;
+    unsigned test_ctas = 0;  // nkg_test_small_run: CTAs whatever the graph's rows are
     DeviceArray<double> y0, y1, part;
     DeviceArray<SmallState> st;
     PinnedHost<SmallState> host;

@@ -2270,8 +2270,10 @@ static void small_setup(nkg_graph *g) {
     for (int c = 0; c < kSmallClasses; ++c)
         P.task[c + 1] = P.task[c] + ceil_div(P.row[c + 2] - P.row[c + 1], 1u << c);
     // One CTA per SM, fewer where each would have less than four warps' tasks.
-    const unsigned ctas = std::max<unsigned>(
+    unsigned ctas = std::max<unsigned>(
         1, std::min<unsigned>(sms, std::max<unsigned>(ceil_div(P.task[kSmallClasses], 4), P.row[1])));
+    if (W.test_ctas)
+        ctas = W.test_ctas;
     W.y0.alloc(n);
     W.y1.alloc(n);
     W.part.alloc(7 * static_cast<size_t>(ctas));
@@ -2280,14 +2282,17 @@ static void small_setup(nkg_graph *g) {
     W.ctas = ctas;
 }
 
+// False where the launch does not fit (a context with part of the SMs) or its
+// grid barrier gave up (CTAs held up by other work): the graph's runs are
+// captured sweeps from then on, which need neither.
 template <typename T>
-static RunResult run_small(nkg_graph *g, const nkg_pr_params &p, const double *d_tele,
-                           double *d_out) {
+static bool run_small(nkg_graph *g, const nkg_pr_params &p, const double *d_tele, double *d_out,
+                      RunResult &R) {
     cudaStream_t s = g->stream;
     SmallWork &W = g->small;
     Plane<T> &P = plane<T>(g);
     const uint32_t n = static_cast<uint32_t>(g->n);
-    RunResult R;
+    R = RunResult{};
     check_cancel(g, "PageRank run cancelled");
     NKG_CUDA(cudaEventRecord(g->ev0, s));
     if (d_tele) {
@@ -2316,7 +2321,7 @@ static RunResult run_small(nkg_graph *g, const nkg_pr_params &p, const double *d
     a.z = g->z;
     a.n = n;
     a.cap = kSmallSweeps;
-    a.polls = kSmallPolls;
+    a.polls = W.polls;
     a.normalized = p.normalized ? 1 : 0;
     const double S0 = static_cast<double>(g->sinks) * a.rp.inv_n;
     a.coef0 = p.distribute_sinks ? (d_tele ? S0 : S0 / static_cast<double>(n)) : 0.0;
@@ -2327,14 +2332,23 @@ static RunResult run_small(nkg_graph *g, const nkg_pr_params &p, const double *d
             NKG_CUDA(cudaMemsetAsync(W.st.get(), 0, sizeof(SmallState), s));
         else
             NKG_CUDA(cudaMemsetAsync(&W.st.get()->barrier, 0, sizeof(unsigned int), s));
-        NKG_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(small_kernel<T>),
-                                             dim3(W.ctas), dim3(kSmallThreads), args, 0, s));
+        const cudaError_t e =
+            cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(small_kernel<T>),
+                                        dim3(W.ctas), dim3(kSmallThreads), args, 0, s);
+        if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorLaunchOutOfResources) {
+            cudaGetLastError();
+            W.declined = true;
+            return false;
+        }
+        NKG_CUDA(e);
         ++R.launches;
         NKG_CUDA(cudaEventRecord(g->ev1, s));
         NKG_CUDA(cudaMemcpyAsync(h, W.st.get(), sizeof(SmallState), cudaMemcpyDeviceToHost, s));
         NKG_CUDA(cudaStreamSynchronize(s));
-        if (h->error)
-            throw Error(NKG_ERR_TIMEOUT, "the grid barrier of the small-graph run timed out");
+        if (h->error) {
+            W.declined = true;
+            return false;
+        }
         if (h->done)
             break;
         check_cancel(g, "PageRank run cancelled");
@@ -2348,7 +2362,7 @@ static RunResult run_small(nkg_graph *g, const nkg_pr_params &p, const double *d
     float ms = 0.f;
     NKG_CUDA(cudaEventElapsedTime(&ms, g->ev0, g->ev1));
     R.ms_total = R.ms_iter = ms;
-    return R;
+    return true;
 }
 
 template <typename T, bool WEIGHTED>
@@ -2356,8 +2370,9 @@ static RunResult run_power(nkg_graph *g, const nkg_pr_params &p, const double *d
                            double *d_out) {
     if (!WEIGHTED && runs_small(g)) {
         small_setup(g);
-        if (g->small.ctas)
-            return run_small<T>(g, p, d_tele, d_out);
+        RunResult R;
+        if (!g->small.declined && run_small<T>(g, p, d_tele, d_out, R))
+            return R;
     }
     cudaStream_t s = g->stream;
     sweep_setup<T, WEIGHTED>(g);
@@ -2783,6 +2798,11 @@ extern "C" {
 const char *nkg_last_error(void) { return nkg::g_last_error.c_str(); }
 
 int nkg_abi_version(void) { return NKG_ABI_VERSION; }
+
+void nkg_test_small_run(nkg_graph *g, uint32_t polls, uint32_t ctas) {
+    g->small.polls = polls;
+    g->small.test_ctas = ctas;
+}
 
 int64_t nkg_test_fail_alloc(int64_t after) {
     const int64_t left = nkg::t_allocs_until_failure;

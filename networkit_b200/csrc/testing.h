@@ -16,6 +16,11 @@ extern "C" {
  * (negative: it has happened, or none was set). */
 NKG_API int64_t nkg_test_fail_alloc(int64_t after);
 
+/* For the one-launch runs of this graph: polls of the grid barrier before it
+ * gives up (0: at once), and the launch's CTAs (0: as many as the graph needs).
+ * Before the handle's first run. */
+NKG_API void nkg_test_small_run(nkg_graph *g, uint32_t polls, uint32_t ctas);
+
 #ifdef __cplusplus
 }
 #endif

@@ -116,3 +116,24 @@ def test_a_row_longer_than_a_ctas_share_is_cut_into_chunks(oracle_mod, hub, one_
     p32 = dg.params(0.85, 0.0, 0, False, True, _capi.NKG_PREC_FP32, 60)
     # FP32 scores of unit mass, one of them most of it: a few roundings of 2^-24
     assert np.abs(dg.run(p32)[0] - o.scores).sum() <= 1e-6
+
+
+@pytest.mark.parametrize("polls,ctas", [(0, 0), (1 << 22, 4096)])
+def test_runs_go_on_as_captured_sweeps_where_one_launch_cannot(polls, ctas):
+    """A grid barrier that gives up at once, and a grid larger than the GPU holds
+    at a time (which the launch refuses): the run is what captured sweeps give."""
+    import ctypes as C
+
+    csr = graph_of_rows([300] * 2000, 20_000, 5)
+    dg, captured = _capi.DeviceGraph(csr), _capi.DeviceGraph(csr, hot_tier_kb=0)
+    f = _capi.lib().nkg_test_small_run
+    f.restype, f.argtypes = None, [C.c_void_p, C.c_uint32, C.c_uint32]
+    f(dg.h, polls, ctas)
+    t = np.random.default_rng(1).random(csr.z)
+    for prec, tele in ((_capi.NKG_PREC_FP64, None), (_capi.NKG_PREC_FP32, None),
+                       (_capi.NKG_PREC_FP64, t / t.sum())):
+        p = dg.params(0.85, 1e-6, 0, False, True, prec, 500)
+        s, it, _, st = dg.run(p, tele)
+        want, want_it, _, want_st = captured.run(p, tele)
+        np.testing.assert_array_equal(s, want)
+        assert it == want_it and st["kernel_launches"] == want_st["kernel_launches"] > 1
