@@ -503,7 +503,8 @@ struct BatchSplit {
 
 struct nkg_batch {
     int device = 0;
-    cudaStream_t stream = nullptr;
+    cudaStream_t stream = nullptr, side = nullptr;  // side: the shared-memory kernel's
+    cudaEvent_t fork = nullptr, join = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     uint32_t count = 0, total = 0;
     uint64_t arcs = 0;
@@ -735,7 +736,7 @@ template <>
 double *smem_buf<double>(nkg_batch *b, int k) { return b->sy64[k].get(); }
 
 template <typename T>
-void smem_launch(nkg_batch *b, double *out) {
+void smem_launch(nkg_batch *b, double *out, cudaStream_t s) {
     const BatchSplit &S = b->splits[sizeof(T) == 8 ? 1 : 0];
     SmemArgs<T> a{};
     a.meta = b->smeta.get();
@@ -756,7 +757,7 @@ void smem_launch(nkg_batch *b, double *out) {
     a.count = S.n_smem;
     cudaLaunchAttribute attr;
     const cudaLaunchConfig_t cfg =
-        smem_config(S.cluster, S.clusters * S.cluster, S.smem_bytes, b->stream, &attr);
+        smem_config(S.cluster, S.clusters * S.cluster, S.smem_bytes, s, &attr);
     NKG_CUDA(cudaLaunchKernelEx(&cfg, batch_smem_kernel<T>, a));
 }
 
@@ -820,10 +821,16 @@ bool batch_launch(nkg_batch *b, const nkg_batch_tuning &t, T *y0, T *y1, double 
             return;
         const BatchSplit &S = b->splits[sizeof(T) == 8 ? 1 : 0];
         NKG_CUDA(cudaMemsetAsync(b->counters.get(), 0, 3 * sizeof(unsigned int), s));
-        if (S.n_smem)
-            smem_launch<T>(b, out);
-        if (!S.n_big)
+        if (!S.n_big) {
+            smem_launch<T>(b, out, s);
             return;
+        }
+        // Both kernels at once, the larger graphs first: they take longest, and
+        // the others fill the SMs that have no more of them.
+        if (S.n_smem) {
+            NKG_CUDA(cudaEventRecord(b->fork, s));
+            NKG_CUDA(cudaStreamWaitEvent(b->side, b->fork, 0));
+        }
         cfg.gridDim = dim3(static_cast<unsigned>(clusters) * t.cluster);
         BatchArgs<T> a{};
         a.meta = b->meta.get();
@@ -846,6 +853,11 @@ bool batch_launch(nkg_batch *b, const nkg_batch_tuning &t, T *y0, T *y1, double 
         a.count = S.n_big;
         a.total = b->total;
         NKG_CUDA(cudaLaunchKernelEx(&cfg, kfn, a));
+        if (S.n_smem) {
+            smem_launch<T>(b, out, b->side);
+            NKG_CUDA(cudaEventRecord(b->join, b->side));
+            NKG_CUDA(cudaStreamWaitEvent(s, b->join, 0));
+        }
     });
     return ok;
 }
@@ -925,8 +937,11 @@ nkg_batch *batch_create(uint32_t count, const uint64_t *node_off, const uint64_t
     b->arcs = arcs;
     b->node_off.assign(node_off, node_off + count + 1);
     b->stream = stream_acquire(dev);
+    b->side = stream_acquire(dev);
     NKG_CUDA(cudaEventCreate(&b->ev0));
     NKG_CUDA(cudaEventCreate(&b->ev1));
+    NKG_CUDA(cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming));
+    NKG_CUDA(cudaEventCreateWithFlags(&b->join, cudaEventDisableTiming));
     cudaStream_t s = b->stream;
     const unsigned sms = num_sms(dev);
 
@@ -1130,13 +1145,13 @@ void nkg_batch_destroy(nkg_batch *b) {
     for (auto &G : b->graphs)
         if (G.exec)
             cudaGraphExecDestroy(G.exec);
-    if (b->ev0)
-        cudaEventDestroy(b->ev0);
-    if (b->ev1)
-        cudaEventDestroy(b->ev1);
-    cudaStream_t s = b->stream;
+    for (cudaEvent_t e : {b->ev0, b->ev1, b->fork, b->join})
+        if (e)
+            cudaEventDestroy(e);
+    cudaStream_t s = b->stream, side = b->side;
     const int dev = b->device;
     delete b;
+    nkg::stream_release(dev, side);
     nkg::stream_release(dev, s);
     if (prev >= 0)
         cudaSetDevice(prev);
