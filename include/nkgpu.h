@@ -293,17 +293,21 @@ NKG_API int nkg_ppr_run(nkg_graph *g, const nkg_pr_params *p, uint32_t k, const 
 
 /* Many-graph batch, no reference counterpart: `count` independent graphs
  * (each PageRank.cpp:20-104 on its own: its own n, teleport (1-damp)/n,
- * residual and stopping test) solved together by one persistent kernel
- * launch, captured in a CUDA graph. The graphs come as one block-diagonal
+ * residual and stopping test) solved together by one or two persistent kernel
+ * launches, captured in a CUDA graph. The graphs come as one block-diagonal
  * in-CSR: graph i owns the node ids [node_offsets[i], node_offsets[i+1]) and
  * every arc stays inside its graph (checked). Unweighted; all nodes exist.
  * FP32 runs stop at tol, at max_iterations, or at the FP32 rounding floor (a
  * residual that shrinks by less than 0.9x in one sweep, which the exact
  * iteration never does); FP64 runs stop at tol or max_iterations.
- * The kernel's launch shape comes from nkg_batch_tuning: thread-block
- * cluster size, threads per CTA, and the row-split threshold (rows longer
- * than `split` arcs are summed by a whole warp, the others one per lane in
- * 32-row slices). nkg_batch_tune times `sweeps` sweeps of every graph for
+ * Graphs whose iterate fits into a CTA's shared memory (57,080 nodes in FP32,
+ * 28,536 in FP64) are run by a kernel whose launch shape the library chooses.
+ * The launch shape of the larger graphs' kernel, which runs beside it, comes
+ * from nkg_batch_tuning: thread-block cluster size, threads per CTA, and the
+ * row-split threshold (rows longer than `split` arcs are summed by a whole
+ * warp, the others one per lane in 32-row slices). nkg_batch_tune (which
+ * times one run, reports it for every candidate and keeps the tuning where
+ * the batch has no larger graph) times `sweeps` sweeps of every graph for
  * each candidate (split 32..1024, 256 or 512 threads, clusters 1..16), or
  * with sweeps = 0 the whole run to convergence under *p (the real objective:
  * it sees the largest graphs' critical path), then the kernel variants on

@@ -43,6 +43,7 @@
 
 #include "common.cuh"
 #include "host.hpp"
+#include "testing.h"
 #include "sweep.cuh"
 
 namespace cg = cooperative_groups;
@@ -526,6 +527,7 @@ struct nkg_batch {
     DeviceArray<uint4> sarcs;
     uint64_t s_entries = 0;                    // entries of their iterates
     bool smem_ready = false;
+    uint32_t smem_most = kNone;                // nodes of their largest (nkg_test_batch_shared)
     DeviceArray<float> sy32[2];
     DeviceArray<double> sy64[2];
     BatchSplit splits[2];                      // [FP32, FP64]
@@ -673,7 +675,7 @@ void batch_split(nkg_batch *b) {
     uint32_t max_n = 0;
     for (uint32_t i : b->order_h) {
         const SmemMeta &m = b->smeta_h[i];
-        if (m.items && m.n <= smem_max_nodes<T>()) {
+        if (m.items && m.n <= std::min(smem_max_nodes<T>(), b->smem_most)) {
             small.push_back(i);
             max_n = std::max(max_n, m.n);
         } else {
@@ -875,28 +877,31 @@ void upload_params(nkg_batch *b, const nkg_pr_params &p) {
                              b->stream));
 }
 
+// The iterates of the kernels that this precision's split uses.
 template <typename T>
 void ensure_iterates(nkg_batch *b);
 template <>
 void ensure_iterates<float>(nkg_batch *b) {
+    const BatchSplit &S = b->splits[0];
     for (auto &y : b->y32)
-        if (!y) {
+        if (S.n_big && !y) {
             y.alloc(static_cast<size_t>(b->total) + 1);
             NKG_CUDA(cudaMemsetAsync(y.get(), 0, (static_cast<size_t>(b->total) + 1) * 4, b->stream));
         }
     for (auto &y : b->sy32)
-        if (!y)
+        if (S.n_smem && !y)
             y.alloc(std::max<uint64_t>(b->s_entries, 4));
 }
 template <>
 void ensure_iterates<double>(nkg_batch *b) {
+    const BatchSplit &S = b->splits[1];
     for (auto &y : b->y64)
-        if (!y) {
+        if (S.n_big && !y) {
             y.alloc(static_cast<size_t>(b->total) + 1);
             NKG_CUDA(cudaMemsetAsync(y.get(), 0, (static_cast<size_t>(b->total) + 1) * 8, b->stream));
         }
     for (auto &y : b->sy64)
-        if (!y)
+        if (S.n_smem && !y)
             y.alloc(std::max<uint64_t>(b->s_entries, 4));
 }
 
@@ -1157,6 +1162,8 @@ void nkg_batch_destroy(nkg_batch *b) {
         cudaSetDevice(prev);
 }
 
+void nkg_test_batch_shared(nkg_batch *b, uint32_t nodes) { b->smem_most = nodes; }
+
 int nkg_batch_get_tuning(const nkg_batch *b, nkg_batch_tuning *t) {
     return guarded([&] {
         require(b != nullptr && t != nullptr, "NULL argument");
@@ -1195,6 +1202,16 @@ int nkg_batch_tune(nkg_batch *b, const nkg_pr_params *p, uint32_t sweeps,
         const uint32_t splits[] = {32, 64, 128, 256, 1024};
         const uint32_t threads[] = {256, 512};
         const uint32_t clusters[] = {1, 2, 4, 8, 16};
+        const bool fp64 = p->precision == NKG_PREC_FP64;
+        auto timed = [&](const nkg_batch_tuning &t) {
+            fp64 ? batch_timed<double>(b, t) : batch_timed<float>(b, t);  // warm-up (layout, caches)
+            return fp64 ? batch_timed<double>(b, t) : batch_timed<float>(b, t);
+        };
+        fp64 ? batch_split<double>(b) : batch_split<float>(b);
+        // Without a graph for batch_kernel every candidate is the same run: timed
+        // once, and the tuning in force is as good as any.
+        const bool shapes = b->splits[fp64 ? 1 : 0].n_big > 0;
+        const float ms_all = shapes ? 0.f : timed(b->tuning);
         nkg_batch_tuning best{};
         best.ms = 1e300;
         uint32_t nres = 0;
@@ -1211,24 +1228,20 @@ int nkg_batch_tune(nkg_batch *b, const nkg_pr_params *p, uint32_t sweeps,
                             : batch_launch<float>(b, t, nullptr, nullptr, nullptr, true);
                     if (!fits)
                         continue;
-                    float ms;
-                    if (p->precision == NKG_PREC_FP64) {
-                        batch_timed<double>(b, t);  // warm-up (layout, caches)
-                        ms = batch_timed<double>(b, t);
-                    } else {
-                        batch_timed<float>(b, t);
-                        ms = batch_timed<float>(b, t);
-                    }
-                    t.ms = ms;
+                    t.ms = shapes ? timed(t) : ms_all;
                     if (results && nres < capacity)
                         results[nres] = t;
                     ++nres;
-                    if (ms < best.ms)
+                    if (t.ms < best.ms)
                         best = t;
                 }
         require(nres > 0, "no cluster shape fits on this GPU");
+        if (!shapes) {
+            best = b->tuning;
+            best.ms = ms_all;
+        }
         // Second stage: the kernel variants on the best shape.
-        for (uint32_t var = 1; var <= 3; ++var) {
+        for (uint32_t var = 1; shapes && var <= 3; ++var) {
             nkg_batch_tuning t = best;
             t.variant = var;
             t.ms = 0.0;
@@ -1238,19 +1251,11 @@ int nkg_batch_tune(nkg_batch *b, const nkg_pr_params *p, uint32_t sweeps,
                     : batch_launch<float>(b, t, nullptr, nullptr, nullptr, true);
             if (!fits)
                 continue;
-            float ms;
-            if (p->precision == NKG_PREC_FP64) {
-                batch_timed<double>(b, t);
-                ms = batch_timed<double>(b, t);
-            } else {
-                batch_timed<float>(b, t);
-                ms = batch_timed<float>(b, t);
-            }
-            t.ms = ms;
+            t.ms = timed(t);
             if (results && nres < capacity)
                 results[nres] = t;
             ++nres;
-            if (ms < best.ms)
+            if (t.ms < best.ms)
                 best = t;
         }
         b->tuning = best;

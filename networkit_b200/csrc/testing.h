@@ -21,6 +21,10 @@ NKG_API int64_t nkg_test_fail_alloc(int64_t after);
  * Before the handle's first run. */
 NKG_API void nkg_test_small_run(nkg_graph *g, uint32_t polls, uint32_t ctas);
 
+/* Graphs of more than `nodes` nodes go to the kernel that nkg_batch_tuning
+ * applies to (0: every graph). Before the handle's first run. */
+NKG_API void nkg_test_batch_shared(nkg_batch *b, uint32_t nodes);
+
 #ifdef __cplusplus
 }
 #endif
