@@ -698,6 +698,7 @@ void batch_split(nkg_batch *b) {
         NKG_CUDA(cudaFuncSetAttribute(
             kfn, cudaFuncAttributeMaxDynamicSharedMemorySize,
             static_cast<int>(smem_launch_bytes<T>(smem_max_nodes<T>()))));
+        NKG_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
         double best = 1e300;
         for (unsigned c = 1; c <= kSmemMaxCluster; c *= 2) {
             cudaLaunchAttribute attr;

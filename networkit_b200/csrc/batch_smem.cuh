@@ -34,7 +34,9 @@ template <typename T>
 constexpr size_t smem_launch_bytes(uint32_t max_n) {
     return (static_cast<size_t>(max_n) + 8) * sizeof(T) / 16 * 16 + 16;
 }
-constexpr int kSmemMaxCluster = 8;
+// 16 CTAs, beyond the portable 8, for batches of few graphs: one of 20,000 nodes
+// and 8M arcs, 60 sweeps, FP64 1.28 ms with 8, 0.71 with 16.
+constexpr int kSmemMaxCluster = 16;
 
 struct SmemMeta {
     uint32_t base;    // first (relabelled) node id

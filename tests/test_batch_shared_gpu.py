@@ -64,3 +64,20 @@ def test_iteration_cap_and_graph_times(batch):
     assert (its == 3).all() and st["iterations"] == 3 * len(gs)
     start, end = db.graph_times()
     assert (start >= 0).all() and (end >= start).all()
+
+
+@pytest.mark.parametrize("prec", [_capi.NKG_PREC_FP64, _capi.NKG_PREC_FP32])
+@pytest.mark.parametrize("count", [1, 3, 20])
+def test_few_graphs_get_larger_clusters(oracle_mod, count, prec):
+    """Up to 16 CTAs a graph, dense ones with hub rows."""
+    gs = [rows_graph([9000, 4000, 300] + [70] * (2500 + 37 * i), 3000 + 41 * i, i)
+          for i in range(count)]
+    csr, offs = concat_in_csr(gs)
+    db = _capi.DeviceBatch(csr, offs)
+    tol = 1e-10 if prec == _capi.NKG_PREC_FP64 else 1e-8
+    s, its, _, st = db.run(_capi.PRParams(0.85, tol, 0, 0, 1, prec, 10000))
+    assert st["kernel_launches"] == 1
+    for i, g in enumerate(gs):
+        o = oracle_mod.pagerank(g, tol=tol, norm=0, distribute_sinks=True)
+        err = float(np.abs(s[int(offs[i]):int(offs[i + 1])] - o.scores).sum())
+        assert err <= (1e-10 if prec == _capi.NKG_PREC_FP64 else 1e-6), (i, err)
