@@ -1351,6 +1351,18 @@ static void build_blocks(SellLayout &L, const BlockPlan &plan, uint32_t n, const
     NKG_CUDA(cudaStreamSynchronize(s));
 }
 
+// L without (a part of) its source blocks.
+static void drop_blocks(SellLayout &L) {
+    L.n_hot = L.n_sums = L.hot_slices = 0;
+    L.hot_steps = 0;
+    L.hot_blocks = HotBlocks{};
+    L.chunk_slot.reset();
+    L.hot_arcs.reset();
+    L.hot_off.reset();
+    L.hot_slot.reset();
+    L.hot_cost.reset();
+}
+
 // Build the sliced layout L of a CSR whose n rows are sorted by length,
 // descending (row_ptr, col, optional weights w through w_index, rowlen).
 void build_sell(SellLayout &L, uint32_t n, const uint32_t *row_ptr, const uint32_t *col,
@@ -1362,13 +1374,20 @@ void build_sell(SellLayout &L, uint32_t n, const uint32_t *row_ptr, const uint32
     const uint32_t arcs = read_scalar(row_ptr + n, s);
     L.chunk = chunk_for(arcs, sms);
     BlockPlan plan{};
-    if (blocks && !w)
-        plan = plan_blocks(n, arcs, row_ptr, col, s);
     DeviceArray<uint32_t> vstart, vlen, pcol, rest;
-    if (plan.blocks && scratch)
-        pcol = std::move(*scratch);
-    if (plan.blocks)
-        build_blocks(L, plan, n, row_ptr, col, rowlen, sms, pcol, rest, vstart, vlen, s);
+    if (blocks && !w) {
+        try {
+            plan = plan_blocks(n, arcs, row_ptr, col, s);
+            if (plan.blocks && scratch)
+                pcol = std::move(*scratch);
+            if (plan.blocks)
+                build_blocks(L, plan, n, row_ptr, col, rowlen, sms, pcol, rest, vstart, vlen, s);
+        } catch (const Error &e) {
+            if (e.code != NKG_ERR_OOM)
+                throw;
+            drop_blocks(L);  // the layout without them needs no scratch of their size
+        }
+    }
     if (!L.n_hot) {
         L.n_chunks = row_chunks(rowlen, n, L.chunk, L.n_long, L.n_vlong, L.chunk_begin, s);
         plain_chunks(L, row_ptr, sms, vstart, vlen, s);

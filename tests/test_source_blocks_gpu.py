@@ -112,3 +112,26 @@ def test_blocked_weights_and_gradients(oracle_mod, rmat):
             vals.append(float(g @ dg.run(dg.params(0.85, 0.0, 0, False, True, 0, 250))[0]))
         fd = (vals[0] - vals[1]) / 2e-4
         assert abs(fd - gw2[e]) <= 1e-4 * abs(gw2[e])
+
+
+def test_blocks_are_left_out_where_memory_is_short(fail_alloc, rmat):
+    """Every allocation of the graph's creation fails in turn: those of the blocks
+    leave a graph without them, the others are the call's error."""
+    csr, dg = rmat
+    p = dg.params(0.85, 1e-9, 0, False, True, _capi.NKG_PREC_FP64, 500)
+    want, want_it = dg.run(p)[:2]
+    plain = 0
+    for k in range(300):
+        fail_alloc(k)
+        try:
+            h = _capi.DeviceGraph(csr)
+        except _capi.NkgError as e:
+            assert e.code == _capi.NKG_ERR_OOM
+            continue
+        if fail_alloc(-1) >= 0:
+            break  # fewer than k + 1 allocations
+        plain += 1
+        s, it = h.run(p)[:2]
+        # another order of summation of the same sweeps
+        assert it == want_it and np.abs(s - want).sum() <= 1e-11
+    assert plain >= 10 and k < 299
