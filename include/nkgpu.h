@@ -391,8 +391,11 @@ NKG_API int nkg_profile_sweeps(nkg_graph *g, int precision, int sweeps, double *
  * sliced layout's column stream in storage order, padding included, read
  * from the current iterate and summed per thread, eight gathers in flight
  * per thread - timed with CUDA events over `reps` launches (after one
- * untimed launch). Its mean launch time is the random-gather bound of this
- * graph on this GPU, the floor under nkg_profile_sweeps' sweep time. */
+ * untimed launch). On a layout without source blocks the mean launch time is
+ * the random-gather bound of this graph on this GPU, the floor under
+ * nkg_profile_sweeps' sweep time; where the library reads the most-used
+ * sources from shared memory, its own kernel for those is timed along with the
+ * bare gathers of the other arcs, and the figure is no bound. */
 NKG_API int nkg_profile_gathers(nkg_graph *g, int precision, int reps, double *ms_gather_kernel);
 
 /* Row partition of the PageRank iteration over several GPUs; no counterpart

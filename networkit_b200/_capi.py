@@ -540,8 +540,8 @@ class DeviceGraph:
         return float(a.value), float(b.value)
 
     def profile_gathers(self, precision: int, reps: int = 20) -> float:
-        """ms per launch of the gathers-only diagnostic kernel (the random
-        gather bound of the sweep on this graph)."""
+        """ms per launch of the gathers-only diagnostic (the random-gather bound
+        of the sweep on a graph whose layout has no source blocks)."""
         a = C.c_double(0.0)
         check(lib().nkg_profile_gathers(self.h, int(precision), int(reps), C.byref(a)))
         return float(a.value)

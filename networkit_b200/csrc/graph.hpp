@@ -67,6 +67,7 @@ struct SellLayout {
     HotBlocks hot_blocks{};
     uint32_t hot_slices = 0;
     uint64_t hot_steps = 0;
+    uint64_t hot_n = 0, hot_sums = 0;   // arcs of the segments, sums of their chunks
     DeviceArray<uint4> hot_arcs;        // 32 lanes x 8 arcs per step
     DeviceArray<uint32_t> hot_off;      // hot_slices + 1
     DeviceArray<uint32_t> hot_slot;     // 32 per slice

@@ -730,14 +730,15 @@ __device__ __forceinline__ uint32_t hot_chunk(const HotBlocks &sl, const HotChun
 // Steps of every hot slice (its first chunk is its longest) and its cost in
 // clocks in FP64 and FP32, fitted to the CTAs' times on R-MAT 22 and 24: 13 a
 // step, 24 a slice, 4.5 (FP32: 2) for every 32 arcs, 20,000 for a change of
-// block. One warp per slice.
+// block; all arcs in *total. One warp per slice.
 __global__ void hot_steps(HotBlocks sl, HotChunks ch, uint32_t slices,
                           const uint32_t *__restrict__ order, const uint32_t *__restrict__ vlen,
                           uint32_t *__restrict__ steps, uint64_t *__restrict__ cost64,
-                          uint64_t *__restrict__ cost32) {
+                          uint64_t *__restrict__ cost32, unsigned long long *__restrict__ total) {
     const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
     const uint32_t lane = threadIdx.x & 31;
+    unsigned long long mine = 0;
     for (uint32_t s = warp; s < slices; s += nwarps) {
         uint32_t b;
         const uint32_t k = hot_chunk(sl, ch, s, lane, b);
@@ -750,8 +751,11 @@ __global__ void hot_steps(HotBlocks sl, HotChunks ch, uint32_t slices,
             steps[s] = n;
             cost64[s] = base + arcs * 9 / 64;
             cost32[s] = base + arcs / 16;
+            mine += arcs;
         }
     }
+    if (mine)
+        atomicAdd(total, mine);
 }
 
 // Arcs and sum slots of the hot slices (one warp each).
@@ -1332,8 +1336,10 @@ static void build_blocks(SellLayout &L, const BlockPlan &plan, uint32_t n, const
     L.hot_off.alloc(static_cast<size_t>(L.hot_slices) + 1);
     L.hot_cost.alloc(2 * static_cast<size_t>(L.hot_slices));
     L.hot_slot.alloc(static_cast<size_t>(L.hot_slices) * 32);
+    DeviceArray<unsigned long long> total(1);
+    NKG_CUDA(cudaMemsetAsync(total.get(), 0, sizeof(unsigned long long), s));
     hot_steps<<<sms * 8, 256, 0, s>>>(L.hot_blocks, ch, L.hot_slices, order, vl, steps.get(),
-                                      cost.get(), cost.get() + L.hot_slices);
+                                      cost.get(), cost.get() + L.hot_slices, total.get());
     NKG_CUDA(cudaGetLastError());
     scan_from_zero(steps.get(), L.hot_off.get(), L.hot_slices, s);
     tb = 0;
@@ -1344,6 +1350,8 @@ static void build_blocks(SellLayout &L, const BlockPlan &plan, uint32_t n, const
         NKG_CUDA(cub::DeviceScan::InclusiveSum(tmp.get(), tb, cost.get() + at, L.hot_cost.get() + at,
                                                static_cast<int64_t>(L.hot_slices), s));
     L.hot_steps = read_scalar(L.hot_off.get() + L.hot_slices, s);
+    L.hot_n = read_scalar(total.get(), s);
+    L.hot_sums = hb[kMaxBlocks];
     L.hot_arcs.alloc(L.hot_steps * 32);
     hot_fill<<<sms * 16, 256, 0, s>>>(L.hot_blocks, ch, L.hot_slices, order, vs, vl, pcol.get(),
                                       L.hot_off.get(), L.hot_slot.get(), L.hot_arcs.get());
@@ -1354,7 +1362,7 @@ static void build_blocks(SellLayout &L, const BlockPlan &plan, uint32_t n, const
 // L without (a part of) its source blocks.
 static void drop_blocks(SellLayout &L) {
     L.n_hot = L.n_sums = L.hot_slices = 0;
-    L.hot_steps = 0;
+    L.hot_steps = L.hot_n = L.hot_sums = 0;
     L.hot_blocks = HotBlocks{};
     L.chunk_slot.reset();
     L.hot_arcs.reset();
@@ -2174,7 +2182,11 @@ static uint64_t bytes_per_sweep(const nkg_graph *g, int elem) {
     // Algorithmic bytes of one sweep: column ids, row offsets, gathered
     // iterate (each value once), previous iterate, new iterate, degree
     // (+ weights and a weighted degree of `elem` bytes for weighted graphs).
-    uint64_t b = 4 * g->arcs + 4 * (g->n + 1) + 3ull * elem * g->n;
+    // Arcs in segments of source blocks are 16-bit ids, and every sum of their
+    // chunks is an index, a store and a load.
+    const SellLayout &L = g->fw;
+    uint64_t b = 4 * (g->arcs - L.hot_n) + 2 * L.hot_n + (4 + 2ull * elem) * L.hot_sums +
+                 4 * (g->n + 1) + 3ull * elem * g->n;
     if (g->weighted)
         b += static_cast<uint64_t>(elem) * g->arcs + static_cast<uint64_t>(elem) * g->n;
     else

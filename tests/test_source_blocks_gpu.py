@@ -14,6 +14,13 @@ pytestmark = pytest.mark.gpu
 THREADS = os.cpu_count() or 1
 
 
+def blocks_of(dg, csr):
+    """Whether the layout has source blocks: a sweep's bytes count their arcs as
+    16-bit ids."""
+    st = dg.run(dg.params(0.85, 0.0, 0, False, False, _capi.NKG_PREC_FP64, 1))[3]
+    return st["bytes_per_sweep_fp64"] < 4 * csr.arcs + 4 * (csr.n + 1) + 28 * csr.n
+
+
 @pytest.fixture(scope="module")
 def rmat():
     """R-MAT 22: large enough for source blocks, hubs of tens of thousands of
@@ -21,6 +28,7 @@ def rmat():
     csr = generators.rmat_directed(22, 18, seed=7)
     dg = _capi.DeviceGraph(csr)
     assert csr.arcs >= 60 << 20  # smaller graphs have none
+    assert blocks_of(dg, csr)
     return csr, dg
 
 
@@ -131,6 +139,7 @@ def test_blocks_are_left_out_where_memory_is_short(fail_alloc, rmat):
         if fail_alloc(-1) >= 0:
             break  # fewer than k + 1 allocations
         plain += 1
+        assert not blocks_of(h, csr)
         s, it = h.run(p)[:2]
         # another order of summation of the same sweeps
         assert it == want_it and np.abs(s - want).sum() <= 1e-11
