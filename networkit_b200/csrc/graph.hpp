@@ -108,11 +108,19 @@ struct HotRun {
     }
 };
 
-// Rows of more than `chunk` arcs cut into chunks of that many in CSR order:
-// their number, those of more than kShortChunks chunks, the first chunk of
-// each (n_long + 1 entries). Returns the number of chunks.
-uint32_t row_chunks(const uint32_t *rowlen, uint32_t n, uint32_t chunk, uint32_t &n_long,
-                    uint32_t &n_vlong, DeviceArray<uint32_t> &chunk_begin, cudaStream_t s);
+// Rows of more than `chunk` arcs (kChunk or kSmallChunk) cut into chunks of that
+// many in CSR order: their number, those of more than kShortChunks chunks, the
+// first chunk of each (n_long + 1 entries). Returns the number of chunks. Where
+// kSmallChunk would split most rows just past their end (rows of 9/8 to 3/2 of it
+// on average, at most kChunk) and the rows alone give 5/6 of the resident lanes a
+// row each, chunk becomes kChunk: the fix-up of those rows then costs more than
+// the shorter lanes save. 40 FP64 iterations, ids in order, split / whole, ms: 80
+// arcs a row 200,000 rows 1.85 / 1.58, 400,000 2.91 / 2.42, 175,000 1.60 / 1.69,
+// 25,000 0.77 / 0.95; 66 arcs, 250,000 rows 1.67 / 1.77; 120 arcs, 200,000 rows
+// 2.05 / 1.95 (FP32 1.56 / 1.69); 160 arcs 2.38 / 2.53.
+uint32_t row_chunks(const uint32_t *rowlen, uint32_t n, uint64_t arcs, unsigned sms,
+                    uint32_t &chunk, uint32_t &n_long, uint32_t &n_vlong,
+                    DeviceArray<uint32_t> &chunk_begin, cudaStream_t s);
 
 // Build the sliced layout of a CSR whose n rows are sorted by length,
 // descending; the weight of entry k is w[w_index[k]] (w[k] without an index,

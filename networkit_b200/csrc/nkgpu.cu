@@ -381,20 +381,20 @@ __global__ void relabel_rows(const uint32_t *__restrict__ perm, const uint64_t *
     }
 }
 
-// Rows longer than `split` arcs (a prefix: the rows are sorted by length, or by
-// length bucket with `split` a power of two), and rows longer than `vsplit`.
-__global__ void count_long(const uint32_t *__restrict__ rowlen, uint64_t n, uint32_t split,
-                           uint64_t vsplit, unsigned long long *__restrict__ cnt) {
+// Rows longer than kSmallChunk and kChunk arcs and, of those, rows of more than
+// kShortChunks chunks (prefixes: the rows are sorted by length, or by length
+// bucket, and the thresholds are powers of two).
+__global__ void count_long(const uint32_t *__restrict__ rowlen, uint64_t n,
+                           unsigned int *__restrict__ cnt) {
+    const uint32_t split[4] = {kSmallChunk, kSmallChunk * kShortChunks, kChunk,
+                               kChunk * kShortChunks};
     const uint64_t r = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x;
-    const bool lg = r < n && rowlen[r] > split;
-    const bool vl = r < n && rowlen[r] > vsplit;
-    const int a = __syncthreads_count(lg);
-    const int b = __syncthreads_count(vl);
-    if (threadIdx.x == 0) {
-        if (a)
-            atomicAdd(cnt, static_cast<unsigned long long>(a));
-        if (b)
-            atomicAdd(cnt + 1, static_cast<unsigned long long>(b));
+    const uint32_t len = r < n ? rowlen[r] : 0u;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int c = __syncthreads_count(len > split[i]);
+        if (threadIdx.x == 0 && c)
+            atomicAdd(cnt + i, static_cast<unsigned int>(c));
     }
 }
 
@@ -1154,24 +1154,23 @@ static void scan_from_zero(const uint32_t *in, uint32_t *out, uint32_t m, cudaSt
     NKG_CUDA(cub::DeviceScan::InclusiveSum(tmp.get(), tb, in, out + 1, static_cast<int64_t>(m), s));
 }
 
-// Rows longer than `split` and rows of more than kShortChunks chunks of `split`.
-static void long_rows(const uint32_t *rowlen, uint32_t n, uint32_t split, uint32_t &n_long,
-                      uint32_t &n_vlong, cudaStream_t s) {
-    DeviceArray<unsigned long long> cnt(2);
-    NKG_CUDA(cudaMemsetAsync(cnt.get(), 0, 2 * sizeof(unsigned long long), s));
-    count_long<<<ceil_div(n, 256), 256, 0, s>>>(
-        rowlen, n, split, static_cast<uint64_t>(split) * kShortChunks, cnt.get());
+uint32_t row_chunks(const uint32_t *rowlen, uint32_t n, uint64_t arcs, unsigned sms,
+                    uint32_t &chunk, uint32_t &n_long, uint32_t &n_vlong,
+                    DeviceArray<uint32_t> &chunk_begin, cudaStream_t s) {
+    DeviceArray<unsigned int> cnt(4);
+    NKG_CUDA(cudaMemsetAsync(cnt.get(), 0, 4 * sizeof(unsigned int), s));
+    count_long<<<ceil_div(n, 256), 256, 0, s>>>(rowlen, n, cnt.get());
     NKG_CUDA(cudaGetLastError());
-    unsigned long long h_cnt[2];
-    NKG_CUDA(cudaMemcpyAsync(h_cnt, cnt.get(), sizeof(h_cnt), cudaMemcpyDeviceToHost, s));
+    unsigned int h[4];
+    NKG_CUDA(cudaMemcpyAsync(h, cnt.get(), sizeof(h), cudaMemcpyDeviceToHost, s));
     NKG_CUDA(cudaStreamSynchronize(s));
-    n_long = static_cast<uint32_t>(h_cnt[0]);
-    n_vlong = static_cast<uint32_t>(h_cnt[1]);
-}
-
-uint32_t row_chunks(const uint32_t *rowlen, uint32_t n, uint32_t chunk, uint32_t &n_long,
-                    uint32_t &n_vlong, DeviceArray<uint32_t> &chunk_begin, cudaStream_t s) {
-    long_rows(rowlen, n, chunk, n_long, n_vlong, s);
+    const uint64_t mean8 = 8 * arcs / n;
+    if (chunk == kSmallChunk && mean8 >= 9 * kSmallChunk && mean8 < 12 * kSmallChunk &&
+        h[0] - h[2] > n / 2 && n / 5 > resident_lanes(sms) / 6)
+        chunk = kChunk;
+    const unsigned int *of = h + (chunk == kSmallChunk ? 0 : 2);
+    n_long = of[0];
+    n_vlong = of[1];
     chunk_begin.alloc(static_cast<size_t>(n_long) + 1);
     if (!n_long) {
         NKG_CUDA(cudaMemsetAsync(chunk_begin.get(), 0, sizeof(uint32_t), s));
@@ -1397,7 +1396,7 @@ void build_sell(SellLayout &L, uint32_t n, const uint32_t *row_ptr, const uint32
         }
     }
     if (!L.n_hot) {
-        L.n_chunks = row_chunks(rowlen, n, L.chunk, L.n_long, L.n_vlong, L.chunk_begin, s);
+        L.n_chunks = row_chunks(rowlen, n, arcs, sms, L.chunk, L.n_long, L.n_vlong, L.chunk_begin, s);
         plain_chunks(L, row_ptr, sms, vstart, vlen, s);
         L.s_chunk = (L.n_chunks + 31) / 32;
     }

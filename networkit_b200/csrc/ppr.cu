@@ -604,8 +604,8 @@ void run_ppr(nkg_graph *g, const nkg_pr_params &p, uint32_t k, const uint32_t *s
         DeviceArray<uint32_t> rowlen(n), begin;
         ppr_row_lengths<<<ceil_div(n, 256), 256, 0, s>>>(g->row_ptr.get(), n, rowlen.get());
         NKG_CUDA(cudaGetLastError());
-        uint32_t vlong = 0;
-        g->rc_chunks = row_chunks(rowlen.get(), n, kChunk, g->rc_long, vlong, begin, s);
+        uint32_t vlong = 0, chunk = kChunk;
+        g->rc_chunks = row_chunks(rowlen.get(), n, g->arcs, sms, chunk, g->rc_long, vlong, begin, s);
         NKG_CUDA(cudaStreamSynchronize(s));
         g->rc_begin = std::move(begin);  // complete, or not there
     }

@@ -41,8 +41,9 @@ namespace nkg {
 // arcs 6.4 / 6.6.
 constexpr uint32_t kChunk = 256;
 constexpr uint32_t kSmallChunk = 64;
+inline uint32_t resident_lanes(unsigned sms) { return sms * 48 * 32; }
 inline uint32_t chunk_for(uint64_t arcs, unsigned sms) {
-    return arcs >= static_cast<uint64_t>(sms) * 48 * 32 * 160 ? kChunk : kSmallChunk;
+    return arcs >= 160ull * resident_lanes(sms) ? kChunk : kSmallChunk;
 }
 // A split row with more chunk sums than this is summed by a whole warp in the
 // fix-up, the others by one thread. With source blocks (hot.cuh) a row has a
