@@ -2242,11 +2242,19 @@ static void upload_run_state(nkg_graph *g, const nkg_pr_params &p, int personal,
 // scores), one launch against the captured sweeps, ms: Erdos-Renyi of 0.3M
 // arcs 0.16 / 0.35, 1.6M 0.27 / 0.50, 6.4M 0.71 / 1.04, 16M 1.58 / 1.81, 48M
 // 4.95 / 4.42; R-MAT of 0.3M arcs 0.77 / 2.43, 6M 2.6 / 4.3, 16M 6.0 / 6.7,
-// 46M 17.6 / 14.4.
+// 46M 17.6 / 14.4. Where ids carry locality, long rows gather from shared lines
+// when neighbouring rows are a warp's lanes, as in the captured sweeps: past
+// kSmallLocalArcs graphs of more than kSmallLocalRow arcs a row stay with them
+// (rows of 80 arcs, arcs within 300 ids, 40 FP64 sweeps: 8M arcs 1.09 / 1.21 ms,
+// 12M 1.51 / 1.39, 16M 1.95 / 1.58; 60 arcs, 15M 1.67 / 1.68).
 constexpr uint64_t kSmallArcs = 20ull << 20;
+constexpr uint64_t kSmallLocalArcs = 10ull << 20;
+constexpr uint32_t kSmallLocalRow = 64;
 static bool runs_small(const nkg_graph *g) {
-    return !g->weighted && g->arcs <= kSmallArcs && g->n <= kSmallArcs && g->sweep_shape == 0 &&
-           g->hot_tier_kb < 0;
+    const bool local = g->row_order == 1 && g->arcs > kSmallLocalArcs &&
+                       g->arcs > kSmallLocalRow * g->n;
+    return !g->weighted && !local && g->arcs <= kSmallArcs && g->n <= kSmallArcs &&
+           g->sweep_shape == 0 && g->hot_tier_kb < 0;
 }
 
 // Class boundaries of the rows: how many are longer than each threshold (a
