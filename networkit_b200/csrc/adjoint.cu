@@ -745,7 +745,7 @@ AdjointState &adjoint_ensure(nkg_graph *g) {
         NKG_CUDA(cudaGetLastError());
         NKG_CUDA(cudaStreamSynchronize(s));
     }
-    build_sell(A->tl, n, A->tptr.get(), tcol.get(), g->weighted ? g->w64src.get() : nullptr,
+    build_sell(A->tl, n, arcs, A->tptr.get(), tcol.get(), g->weighted ? g->w64src.get() : nullptr,
                A->tarc.get(), A->tdegc.get(), g->device, s);
     if (g->weighted) {
         A->w_sell32.alloc(A->tl.slots, 4);

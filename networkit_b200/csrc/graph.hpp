@@ -128,8 +128,8 @@ uint32_t row_chunks(const uint32_t *rowlen, uint32_t n, uint64_t arcs, unsigned 
 // entry of an iterate of n + 1). `blocks`: unweighted, columns numbered as the
 // rows are; the layout may get source blocks. `scratch`: an array of `arcs`
 // entries that is no longer needed, or null.
-void build_sell(SellLayout &L, uint32_t n, const uint32_t *row_ptr, const uint32_t *col,
-                const double *w, const uint32_t *w_index, const uint32_t *rowlen, int device,
+void build_sell(SellLayout &L, uint32_t n, uint64_t arcs, const uint32_t *row_ptr,
+                const uint32_t *col, const double *w, const uint32_t *w_index, const uint32_t *rowlen, int device,
                 cudaStream_t s, uint32_t pad_col = kNone, bool blocks = false,
                 DeviceArray<uint32_t> *scratch = nullptr);
 // map[slot] = index[k] for the CSR entry k each slot of L holds (kNone for

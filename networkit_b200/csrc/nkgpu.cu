@@ -1372,13 +1372,12 @@ static void drop_blocks(SellLayout &L) {
 
 // Build the sliced layout L of a CSR whose n rows are sorted by length,
 // descending (row_ptr, col, optional weights w through w_index, rowlen).
-void build_sell(SellLayout &L, uint32_t n, const uint32_t *row_ptr, const uint32_t *col,
-                const double *w, const uint32_t *w_index, const uint32_t *rowlen, int device,
+void build_sell(SellLayout &L, uint32_t n, uint64_t arcs, const uint32_t *row_ptr,
+                const uint32_t *col, const double *w, const uint32_t *w_index, const uint32_t *rowlen, int device,
                 cudaStream_t s, uint32_t pad_col, bool blocks, DeviceArray<uint32_t> *scratch) {
     if (pad_col == kNone)
         pad_col = n;
     const unsigned sms = num_sms(device);
-    const uint32_t arcs = read_scalar(row_ptr + n, s);
     L.chunk = chunk_for(arcs, sms);
     BlockPlan plan{};
     DeviceArray<uint32_t> vstart, vlen, pcol, rest;
@@ -1687,7 +1686,7 @@ static nkg_graph *build_graph(std::unique_ptr<nkg_graph> g, DeviceArray<uint64_t
         if (opt->arc_order == 1 && arcs > 1 && arcs < 0x7fffffffull)
             sort_rows(g.get(), s);
     }
-    build_sell(g->fw, static_cast<uint32_t>(n), g->row_ptr.get(), g->col.get(), g->w64src.get(),
+    build_sell(g->fw, static_cast<uint32_t>(n), arcs, g->row_ptr.get(), g->col.get(), g->w64src.get(),
                nullptr, rowlen.get(), dev, s, kNone, true, &d_col);
     NKG_CUDA(cudaEventRecord(g->ev1, s));
     NKG_CUDA(cudaStreamSynchronize(s));

@@ -254,7 +254,7 @@ nkg_part *create_part(uint64_t vec_len, uint64_t row_base, uint64_t rows, uint64
                                             p->row_map.get(), new_ptr.get(), n, new_col.get(),
                                             w ? new_w.get() : nullptr);
     NKG_CUDA(cudaGetLastError());
-    build_sell(p->fw, n, new_ptr.get(), new_col.get(), w ? new_w.get() : nullptr, nullptr,
+    build_sell(p->fw, n, arcs, new_ptr.get(), new_col.get(), w ? new_w.get() : nullptr, nullptr,
                len.get(), dev, s, pad);
 
     // Launch shape of the regular sweep (512 threads, 8 gathers in flight),
