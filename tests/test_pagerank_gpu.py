@@ -106,11 +106,11 @@ def test_er_config_parity(oracle_mod):
 
 @pytest.mark.parametrize("n, deg", [(100_000, 10), (400_000, 8)])
 def test_graphs_without_split_rows(oracle_mod, n, deg):
-    """Graphs with no row over 256 arcs: the smaller one has few enough work
-    units that the sweep's last CTA closes every iteration (no fix-up
-    launch); the larger one has more than 8,192 units, so a fix-up with no
-    split rows adds the units' partials. Both against the oracle, with and
-    without distributeSinks, and bit-identical on a second run."""
+    """Graphs with no row over 256 arcs, below and above the 8,192 work units
+    where the captured sweeps close an iteration differently, against the
+    oracle, with and without distributeSinks, and bit-identical on a second
+    run. (Graphs of this size run in one launch by default; the captured
+    sweeps without split rows are in test_split_rows_gpu.py.)"""
     csr = generators.erdos_renyi(n, deg / (n - 1), seed=5)
     assert int(np.diff(csr.in_ptr.astype(np.int64)).max()) <= 256
     slices = (n + 31) // 32

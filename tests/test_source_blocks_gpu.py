@@ -1,13 +1,15 @@
-"""Layouts whose long rows are grouped by source blocks (graphs of a few million
-arcs whose leading sources are gathered most) against the oracle: the plain and
-the centrality sweeps, the FP32 solve, weights and their gradients, and
-personalised PageRank, which reads the CSR itself."""
+"""Layouts whose long rows are grouped by source blocks (unweighted graphs of 60 Mi
+arcs and more whose leading sources are gathered most) against the oracle: the
+plain and the centrality sweeps, the FP32 forms, every order of rows and arcs, a
+last block of few ids; and on graphs of that size what has no blocks: weights and
+their gradients, and personalised PageRank, which reads the CSR itself."""
 import os
 
 import numpy as np
 import pytest
 
 from networkit_b200 import _capi, generators
+from networkit_b200.graph import InCSR
 
 pytestmark = pytest.mark.gpu
 
@@ -68,6 +70,50 @@ def test_fp32_rows_of_many_segments_round_like_their_epilogue(rmat):
     assert np.sqrt((rel * rel).mean()) <= np.sqrt(4 / 3) * 0.72
 
 
+@pytest.fixture(scope="module")
+def rmat_scores(oracle_mod, rmat):
+    return oracle_mod.pagerank(rmat[0], tol=1e-10, norm=0, distribute_sinks=True, nthreads=THREADS)
+
+
+def close_to(dg, o):
+    """FP64, FP32 and refined runs against FP64 scores of the oracle (tol 1e-10)."""
+    p = dg.params(0.85, 1e-10, 0, False, True, _capi.NKG_PREC_FP64, 5000)
+    s, it, _, _ = dg.run(p)
+    assert abs(it - o.iterations) <= 1 and np.abs(s - o.scores).sum() <= 1e-10
+    p32 = dg.params(0.85, 0.0, 0, False, True, _capi.NKG_PREC_FP32, 60)
+    # FP32 scores of unit mass: a few roundings of 2^-24 each
+    assert np.abs(dg.run(p32)[0] - o.scores).sum() <= 2e-6
+    p.precision = _capi.NKG_PREC_FP32_REFINE
+    # both stop at a residual of 1e-10, at most 1e-10 / (1 - 0.85) from the fixed point
+    assert np.abs(dg.run(p)[0] - o.scores).sum() <= 2e-9
+
+
+@pytest.mark.parametrize("options", [dict(row_order=1), dict(row_order=0), dict(arc_order=1),
+                                     dict(hot_tier_kb=64), dict(hot_tier_kb=200),
+                                     dict(sweep_shape=2)], ids=str)
+def test_every_layout_option_with_blocks(rmat, rmat_scores, options):
+    dg = _capi.DeviceGraph(rmat[0], **options)
+    assert blocks_of(dg, rmat[0])
+    close_to(dg, rmat_scores)
+
+
+@pytest.mark.parametrize("n", [3 * 24576 + 1, 2 * 24576 + 3, 24576 + 24575])
+def test_a_last_block_of_few_ids(oracle_mod, n):
+    """Dense graphs whose last block of 24,576 sources has one id, three (no whole
+    16 bytes) and all but one."""
+    rng = np.random.default_rng(n)
+    arcs = 64 << 20
+    lens = rng.multinomial(arcs, rng.dirichlet(np.full(n, 3.0)))
+    src = rng.integers(0, n, arcs, dtype=np.uint32)
+    out = np.bincount(src, minlength=n)
+    csr = InCSR(n, n, np.concatenate([[0], np.cumsum(lens)]).astype(np.uint64), src, None,
+                out.astype(np.float64), out.astype(np.uint32), None, True)
+    dg = _capi.DeviceGraph(csr)
+    assert blocks_of(dg, csr)
+    close_to(dg, oracle_mod.pagerank(csr, tol=1e-10, norm=0, distribute_sinks=True,
+                                     nthreads=THREADS))
+
+
 def test_blocked_centralities_match_oracle(oracle_mod, rmat):
     csr, dg = rmat
     s, it, _ = dg.eigenvector(1e-9)
@@ -80,7 +126,7 @@ def test_blocked_centralities_match_oracle(oracle_mod, rmat):
     assert np.abs(s - o).sum() <= 1e-10 * np.abs(o).sum()
 
 
-def test_blocked_ppr_columns_match_the_fp64_run(rmat):
+def test_ppr_columns_match_the_fp64_run_with_blocks(rmat):
     csr, dg = rmat
     seeds = np.array([5, 1 << 21, 77], np.uint32)
     p = dg.params(0.85, 1e-8, 0, False, True, _capi.NKG_PREC_FP32, 300)
@@ -92,7 +138,7 @@ def test_blocked_ppr_columns_match_the_fp64_run(rmat):
         assert np.abs(got[j] - dg.run(p64, t)[0]).sum() <= 1e-6
 
 
-def test_blocked_weights_and_gradients(oracle_mod, rmat):
+def test_weighted_graph_of_that_size_and_its_gradients(oracle_mod, rmat):
     a = generators.with_uniform_weights(rmat[0], seed=3)
     b = generators.with_uniform_weights(rmat[0], seed=4)
     dg, ref = _capi.DeviceGraph(a), _capi.DeviceGraph(b)

@@ -1,6 +1,7 @@
-"""Rows of many chunks, whose chunk sums a warp or (past 2,048 of them) a whole
-CTA adds: the captured sweeps, weights, centralities and the adjoint, whose
-split rows are the out-rows."""
+"""The captured sweeps and their split rows: rows of many chunks, whose chunk sums
+a warp or (past 2,048 of them) a whole CTA adds, in the sweeps, with weights, in
+the centralities and in the adjoint, whose split rows are the out-rows; no split
+rows at all; and a graph between the sizes of one launch and of source blocks."""
 import os
 
 import numpy as np
@@ -82,3 +83,39 @@ def test_split_rows_of_the_adjoint(graph):
             dg.set_weights(w)
             vals.append(float(g @ dg.run(f)[0]))
         assert abs((vals[0] - vals[1]) / 2e-4 - gw[e]) <= 1e-4 * abs(gw[e])
+
+
+@pytest.mark.parametrize("n, deg", [(100_000, 10), (400_000, 8)])
+def test_captured_sweeps_without_split_rows(oracle_mod, n, deg):
+    """Few enough work units that the sweep's last CTA closes every iteration (one
+    launch a sweep), and more than 8,192, so that a fix-up without split rows adds
+    the units' partials (two launches)."""
+    csr = generators.erdos_renyi(n, deg / (n - 1), seed=5)
+    dg = _capi.DeviceGraph(csr, hot_tier_kb=0)
+    assert dg.info()["split_rows"] == 0
+    for distribute in (False, True):
+        o = oracle_mod.pagerank(csr, tol=1e-10, norm=0, distribute_sinks=distribute)
+        p = dg.params(0.85, 1e-10, 0, False, distribute, _capi.NKG_PREC_FP64, 5000)
+        s, it, _, st = dg.run(p)
+        assert abs(it - o.iterations) <= 1 and np.abs(s - o.scores).sum() <= 1e-10
+        np.testing.assert_array_equal(dg.run(p)[0], s)
+        # batches of 2, 4, 8, 8, ... captured graphs of 8 sweeps, three launches beside
+        sweeps = [16, 48, 112, 176, 240]
+        took = next(k for k in sweeps if k >= it)
+        assert st["kernel_launches"] == took * (1 if n == 100_000 else 2) + 3
+
+
+def test_graph_past_one_launch_and_below_source_blocks(oracle_mod):
+    csr = generators.rmat_directed(21, 16, seed=4)
+    assert 20 << 20 < csr.arcs < 60 << 20
+    dg = _capi.DeviceGraph(csr)
+    o = oracle_mod.pagerank(csr, tol=1e-10, norm=0, distribute_sinks=True, nthreads=THREADS)
+    p = dg.params(0.85, 1e-10, 0, False, True, _capi.NKG_PREC_FP64, 5000)
+    s, it, _, st = dg.run(p)
+    assert st["kernel_launches"] > 1
+    assert st["bytes_per_sweep_fp64"] == 4 * csr.arcs + 4 * (csr.n + 1) + 28 * csr.n  # no blocks
+    assert abs(it - o.iterations) <= 1 and np.abs(s - o.scores).sum() <= 1e-10
+    p.precision = _capi.NKG_PREC_FP32_REFINE
+    assert np.abs(dg.run(p)[0] - o.scores).sum() <= 2e-9
+    p32 = dg.params(0.85, 0.0, 0, False, True, _capi.NKG_PREC_FP32, 60)
+    assert np.abs(dg.run(p32)[0] - o.scores).sum() <= 2e-6
