@@ -120,9 +120,13 @@ typedef struct {
                             gathers in flight per lane (-1 default = 0: 512
                             threads, 8; 1: 256, 8; 2: 256, 4; 3: 256, 16) */
     int32_t arc_order;   /* 0 (default): keep every in-row in the caller's order,
-                            which is the reference's summation order; 1: sort
-                            each in-row by source after relabelling (faster
-                            gathers, sums rounded in a different order) */
+                            which is the reference's; 1: sort each in-row by
+                            source after relabelling (faster gathers). Rows are
+                            summed in that order, except that long rows are
+                            summed in chunks, unweighted graphs of at most 20 Mi
+                            arcs by several lanes a row, and unweighted ones from
+                            60 Mi arcs by blocks of sources: in a fixed order
+                            too, but rounded differently */
     int32_t row_order;   /* relabelling of the rows for the sliced layout: 0 (default)
                             in-degree, descending; 1 half-octave in-degree buckets,
                             descending, keeping the caller's id order inside a bucket

@@ -30,7 +30,8 @@
 
 namespace nkg {
 
-// Sources per block: the largest multiple of 4,096 whose FP64 values fit.
+// Sources per block: 192 KB of FP64 values, 96 KB of FP32 ones (28,672, the next
+// multiple of 4,096, would still fit in FP64).
 constexpr uint32_t kHotIds = 24576;
 constexpr uint32_t kMaxBlocks = 31;
 // A block is worth while where at least this many arcs, and this share of all,

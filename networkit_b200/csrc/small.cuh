@@ -20,7 +20,8 @@
 // Every CTA's residual and sink partials go to a slot per CTA; after the
 // barrier every CTA adds all slots in the same order and takes the same
 // decision, while its other warps already gather for the next sweep. Runs are
-// bit-reproducible.
+// bit-reproducible. Where the grid does not fit or the barrier gives up, the
+// run is made by the captured sweeps instead.
 #pragma once
 
 #include "common.cuh"

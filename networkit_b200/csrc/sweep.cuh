@@ -13,11 +13,11 @@
 // Layout (SELL-C-sigma, Kreutzer et al., SIAM J. Sci. Comput. 36(5), 2014, with
 // C = 32 and sigma = n): nodes are relabelled by in-degree, descending, so 32
 // consecutive rows have nearly equal length. Rows longer than kChunk arcs are
-// cut into chunks of kChunk arcs ("virtual rows", placed first); of rows with
-// source blocks (hot.cuh) only the arcs outside the blocks are here. Slice s holds
+// cut into chunks of kChunk arcs ("virtual rows", placed first; kSmallChunk in
+// graphs of fewer arcs); of rows with source blocks (hot.cuh) only the arcs outside the blocks are here. Slice s holds
 // 32 virtual rows column-major: slot (j, lane) at col_sell[(off[s] + j) * 32 +
 // lane], so a warp loads 128 contiguous bytes per step and every lane sums its
-// own row sequentially, in the reference's arc order. No shared memory and no
+// own row sequentially, in the caller's arc order. No shared memory and no
 // barriers are needed: the whole L1 is left to cache the hot part of y.
 // The slices are cut into contiguous, cost-balanced ranges ("units", fixed at
 // set-up). Every warp runs one unit of its own first and then takes the next
@@ -255,8 +255,8 @@ __device__ __forceinline__ void finish_row_sweep(const SweepArgs<T> &a, uint32_t
 // shared memory, so the whole L1 caches the hot scores. The sweep is bound by
 // L1 miss requests to L2 (one sector per scattered lane). Measured
 // alternatives that were slower on B200: L2-only loads; holding the hottest
-// scores in shared memory (random 8-byte loads hit bank conflicts and
-// throttle the MIO queue); per-lane L1 evict-last / no-allocate hints (the
+// scores in the shared memory of this kernel, beside its other gathers (a kernel
+// that gathers from shared memory only is hot.cuh); per-lane L1 evict-last / no-allocate hints (the
 // predicated loads raise register use and cut occupancy).
 
 // Launch shapes of the sweep kernel: threads per CTA and slot steps per batch

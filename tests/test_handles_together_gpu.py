@@ -43,25 +43,57 @@ def test_tier_graph_runs_again_after_a_smaller_tier():
         assert np.abs(large.run(p, t)[0] - small.run(p, t)[0]).sum() <= 2e-9
 
 
-def test_wide_ppr_on_two_threads():
-    csr = generators.rmat_directed(12, 16, seed=5)
-    ks = (256, 130)  # 192 and 215 KB of shared memory
-    handles = [_capi.DeviceGraph(csr) for _ in ks]
-    seeds = [np.arange(k, dtype=np.uint32) for k in ks]
-    p = handles[0].params(0.85, 1e-7, 0, False, True, F32, 100)
-    want = [h.ppr(s, p)[0] for h, s in zip(handles, seeds)]
+def on_two_threads(calls):
+    """Each call on a thread of its own, at the same time; their errors."""
     errors = []
 
-    def work(i):
+    def work(call):
         try:
-            for _ in range(40):
-                np.testing.assert_array_equal(handles[i].ppr(seeds[i], p)[0], want[i])
+            call()
         except BaseException as e:  # handed to the test's own thread
             errors.append(e)
 
-    threads = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+    threads = [threading.Thread(target=work, args=(c,)) for c in calls]
     for t in threads:
         t.start()
     for t in threads:
         t.join()
     assert not errors, errors
+
+
+def test_wide_ppr_on_two_threads():
+    csr = generators.rmat_directed(12, 16, seed=5)
+    ks = (256, 130)
+    handles = [_capi.DeviceGraph(csr) for _ in ks]
+    seeds = [np.arange(k, dtype=np.uint32) for k in ks]
+    p = handles[0].params(0.85, 1e-7, 0, False, True, F32, 100)
+    want = [h.ppr(s, p)[0] for h, s in zip(handles, seeds)]
+
+    def again(i):
+        for _ in range(40):
+            np.testing.assert_array_equal(handles[i].ppr(seeds[i], p)[0], want[i])
+
+    on_two_threads([lambda: again(0), lambda: again(1)])
+
+
+def test_one_launch_runs_and_batches_on_two_threads():
+    """Whole-GPU launches (a grid barrier, clusters) of different streams."""
+    g = _capi.DeviceGraph(generators.rmat_directed(17, 16, seed=6))
+    b = er_batch(20000, 4)
+    g2 = _capi.DeviceGraph(generators.rmat_directed(16, 16, seed=7))
+    pg = g.params(0.85, 1e-9, 0, False, True, F64, 500)
+    pb = _capi.PRParams(0.85, 1e-8, 0, 0, 0, F32, 1000)
+    want, launches = g.run(pg)[0], g.run(pg)[3]["kernel_launches"]
+    want2, want_b = g2.run(pg)[0], b.run(pb)[0]
+    assert launches == 1
+
+    def graph(h, w):
+        for _ in range(60):
+            np.testing.assert_array_equal(h.run(pg)[0], w)
+
+    def batch():
+        for _ in range(60):
+            np.testing.assert_array_equal(b.run(pb)[0], want_b)
+
+    on_two_threads([lambda: graph(g, want), lambda: graph(g2, want2)])
+    on_two_threads([lambda: graph(g, want), batch])
