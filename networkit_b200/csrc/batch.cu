@@ -943,11 +943,8 @@ nkg_batch *batch_create(uint32_t count, const uint64_t *node_off, const uint64_t
     b->arcs = arcs;
     b->node_off.assign(node_off, node_off + count + 1);
     b->stream = stream_acquire(dev);
-    b->side = stream_acquire(dev);
     NKG_CUDA(cudaEventCreate(&b->ev0));
     NKG_CUDA(cudaEventCreate(&b->ev1));
-    NKG_CUDA(cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming));
-    NKG_CUDA(cudaEventCreateWithFlags(&b->join, cudaEventDisableTiming));
     cudaStream_t s = b->stream;
     const unsigned sms = num_sms(dev);
 
@@ -1057,6 +1054,9 @@ nkg_batch *batch_create(uint32_t count, const uint64_t *node_off, const uint64_t
     b->tuning.threads = 256;
     b->tuning.split = 128;
     NKG_CUDA(cudaStreamSynchronize(s));
+    NKG_CUDA(cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming));
+    NKG_CUDA(cudaEventCreateWithFlags(&b->join, cudaEventDisableTiming));
+    b->side = stream_acquire(dev);
     return b.release();
 }
 
