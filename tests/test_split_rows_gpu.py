@@ -119,3 +119,27 @@ def test_graph_past_one_launch_and_below_source_blocks(oracle_mod):
     assert np.abs(dg.run(p)[0] - o.scores).sum() <= 2e-9
     p32 = dg.params(0.85, 0.0, 0, False, True, _capi.NKG_PREC_FP32, 60)
     assert np.abs(dg.run(p32)[0] - o.scores).sum() <= 2e-6
+
+
+@pytest.mark.parametrize("n,reach,whole", [(150_000, 150, False), (200_000, 150, True)])
+def test_long_rows_of_local_ids(oracle_mod, n, reach, whole):
+    """Rows of 80 arcs to nearby ids, 12M and 16M arcs: captured sweeps, not one
+    launch, and with a row for nearly every resident lane the rows stay whole
+    although they are longer than a chunk of 64."""
+    rng = np.random.default_rng(n)
+    lens = rng.integers(70, 91, n)
+    dst = np.repeat(np.arange(n), lens)
+    src = ((dst + rng.integers(1, reach, dst.size)) % n).astype(np.uint32)
+    out = np.bincount(src, minlength=n)
+    csr = InCSR(n, n, np.concatenate([[0], np.cumsum(lens)]).astype(np.uint64), src, None,
+                out.astype(np.float64), out.astype(np.uint32), None, True)
+    dg = _capi.DeviceGraph(csr)
+    info = dg.info()
+    assert info["row_order"] == 1 and (info["split_rows"] == 0) == whole
+    o = oracle_mod.pagerank(csr, tol=1e-10, norm=0, distribute_sinks=True, nthreads=THREADS)
+    p = dg.params(0.85, 1e-10, 0, False, True, _capi.NKG_PREC_FP64, 5000)
+    s, it, _, st = dg.run(p)
+    assert st["kernel_launches"] > 1
+    assert abs(it - o.iterations) <= 1 and np.abs(s - o.scores).sum() <= 1e-10
+    s2 = _capi.DeviceGraph(csr, row_order=0).run(p)[0]  # one launch
+    assert np.abs(s2 - o.scores).sum() <= 1e-10
